@@ -1,10 +1,11 @@
 // The tile rasterizer (INRIA renderCUDA; the reference's shaders/tile_render.comp:281-400 and
 // the CPU reference's per-pixel loop, src/splat/reference_renderer.cpp:120-222).
 //
-// One 256-thread block per 16x16 tile, one thread per pixel; warp w owns an 8 x 4 pixel block.
-// The tile's entries [ranges[tile].x, ranges[tile].y) are walked front to back in batches of
-// 256 records, double-buffered: while batch b is blended, the records of batch b+1 are gathered
-// into shared memory with cp.async (16-byte LDGSTS, the record of gaussian values[j]). Each
+// One 128-thread block per 16x16 tile, two neighbouring pixels a thread; warp w owns an 8 x 8 pixel
+// block. (The window, the stats build and 8 x 8 tiles: one pixel a thread, 8 x 4 blocks.) The tile's
+// entries [ranges[tile].x, ranges[tile].y) are walked front to back in batches of one record a
+// thread: while batch b is blended, the records of batch b+1 are gathered into shared memory with
+// cp.async (16-byte LDGSTS, the record of gaussian values[j], each thread its own). Each
 // entry is then prepared once per block: its power, in base 2 and with log2(opacity) added,
 // expanded as a quadratic in the pixel's offset from the centre of its 32 x 16 cell (powerAt), so that
 //   alpha = min(0.99, 2^p) = min(0.99, o * exp(power))
@@ -15,6 +16,11 @@
 //   skip power > 0; skip alpha < 1/255; testT = T (1 - alpha); testT < 1e-4 -> done;
 //   C += colour alpha T; T = testT
 // and a whole-tile vote (__syncthreads_count) ends the tile once every pixel is done.
+//
+// Bound by instruction issue (77 % of the slots, 160 M warp instructions a 1080p view against 210 M
+// with one pixel a thread and a branch per test): blendPair spends ten predicated instructions a
+// pair, and groups of records that can reach neither the 0.99 cap nor a positive power (nearly all)
+// skip those two tests.
 //
 // Tiles are the frame's tiles over all of its views (DevView): tile t belongs to the view whose
 // [tileBase, tileBase + tilesX * tilesY) holds it, the records of that view's gaussians are at
@@ -29,6 +35,8 @@
 // image within 1/255. The image does not depend on the tile shape, the schedule or the gather.
 #include <cuda.h>  // CUtensorMap (the type only; maps are encoded by the host)
 
+#include <type_traits>
+
 #include "gsr_device.cuh"
 #include "kernels.cuh"
 #include "render_splat.cuh"
@@ -38,6 +46,10 @@ namespace gsr {
 namespace {
 
 constexpr int kRenderThreads = 256;
+constexpr int kHitGroup = 2;  // hits of a warp's list taken together (4: 0.199 against 0.196 ms at 1080p)
+// Threads resident on a SM without the window: 64 registers each (1080p 0.199 ms; 1,152 threads at
+// 56 registers 0.205, 1,280 at 48 registers 0.212).
+constexpr int kResidentThreads = 1024;
 constexpr int kPersistentBlocksPerSm = 4;
 constexpr uint32_t kRenderQueueTicket = 13;  // DeviceControl::tickets slot of the persistent queue
 constexpr float kMaxAlpha = 0.99f;
@@ -71,8 +83,19 @@ __device__ __forceinline__ float approxSqrt(float x) {
 __host__ __device__ constexpr int tileW(int code) { return code; }
 __host__ __device__ constexpr int tileH(int code) { return code == 32 ? 8 : code; }
 __host__ __device__ constexpr int tilePixels(int code) { return tileW(code) * tileH(code); }
+// Pixels a thread owns, neighbours in a row. Two: what depends on the record or on the row alone (its
+// loads, the hit list, three of the power's FMAs) is paid once for both, and a tile needs half the
+// warps and strips. 1080p render pass 0.248 -> 0.196 ms, 24 uneven views 2.79 -> 1.87 ms, 4K 1.156
+// -> 0.873 ms. One pixel in 8 x 8 tiles (one warp a tile would have nothing to hide its latency),
+// with the window (its slots fill the registers) and in the stats build (its counts are a lane's).
+__host__ __device__ constexpr int pixelsPerThread(int cap, int code, bool stats) {
+    return cap == 0 && code != 8 && !stats ? 2 : 1;
+}
+__host__ __device__ constexpr int tileThreads(int cap, int code, bool stats) {
+    return tilePixels(code) / pixelsPerThread(cap, code, stats);
+}
 
-// The warp strips (8 x 4 pixel blocks of a tile; bit w = warp w's) that a record's
+// The warp strips (8 x 4 PX pixel blocks of a tile; bit w = warp w's) that a record's
 // cutoff ellipse q(d) = A dx^2 + 2B dx dy + C dy^2 <= t meets, computed once per record. At
 // distance dy = cy - y from the centre the ellipse's run is cx + (B/A) dy -/+ sqrt((t - (D/A) dy^2)
 // / A); over a strip row's y-range its right edge (concave in dy) peaks at the ellipse's
@@ -80,10 +103,10 @@ __host__ __device__ constexpr int tilePixels(int code) { return tileW(code) * ti
 // point. The test keeps the margins of the tile-coverage box: t + 0.2 %, the y-range widened by
 // 0.05 px, the run by 0.1 % + 0.05 px, over a continuous y-range (a superset of the pixel rows),
 // so a strip holding a pixel with alpha >= 1/255 is always set; a NaN sets the strip.
-template <int TILE>
+template <int TILE, int PX>
 __device__ __forceinline__ uint32_t stripMask(float cx, float cy, float A, float B, float C, float D, float t,
                                               float tileX, float tileY) {
-    constexpr uint32_t kStripsX = tileW(TILE) / 8, kGroups = tileH(TILE) / 4;
+    constexpr uint32_t kRows = 4 * PX, kStripsX = tileW(TILE) / 8, kGroups = tileH(TILE) / kRows;
     const float tt = t * 1.002f;
     const float ia = 1.0f / A, bA = B * ia, dA = D * ia;
     const float ey = approxSqrt(tt / dA);
@@ -91,7 +114,7 @@ __device__ __forceinline__ uint32_t stripMask(float cx, float cy, float A, float
     uint32_t mask = 0;
 #pragma unroll
     for (uint32_t g = 0; g < kGroups; ++g) {
-        const float ya = tileY + float(4 * g) - 0.05f, yb = tileY + float(4 * g + 3) + 0.05f;
+        const float ya = tileY + float(kRows * g) - 0.05f, yb = tileY + float(kRows * g + kRows - 1) + 0.05f;
         const float lo = fmaxf(cy - yb, -ey), hi = fminf(cy - ya, ey);  // dy range inside the ellipse
         if (lo > hi) continue;
         const float dr = fminf(fmaxf(dyR, lo), hi), dl = fminf(fmaxf(-dyR, lo), hi);
@@ -107,11 +130,12 @@ __device__ __forceinline__ uint32_t stripMask(float cx, float cy, float A, float
     return mask;
 }
 
-// 32 x 8 tiles: the strips (bit g * 4 + c: columns 8c .. 8c + 7 of the tile, either row group)
+// 32 x 8 tiles: the strips (bit g * 4 + c: columns 8c .. 8c + 7 of the tile, every row group)
 // inside the splat's 16-px tile rectangle along x, [16 minX, 16 maxX) with the preprocess's
 // tileRect arithmetic (its upper clamp to the grid only removes pixels past the image). The
 // rectangle's edges are multiples of 16 and the strips' multiples of 8, so a strip is wholly in
 // or out. (Along y the tile's 8 rows always lie inside or outside the rectangle's 16-px rows.)
+template <int PX>
 __device__ __forceinline__ uint32_t rectStrips32(float cx, float radius, uint32_t tileX) {
     const float fr = float(ftoi(radius));
     const int x0 = 16 * imax(0, ftoi((cx - fr) / float(kTileSize)));
@@ -120,22 +144,26 @@ __device__ __forceinline__ uint32_t rectStrips32(float cx, float radius, uint32_
 #pragma unroll
     for (uint32_t c = 0; c < 4; ++c) {
         const int s = int(tileX + 8 * c);
-        if (s >= x0 && s < x1) m |= 0x11u << c;
+        if (s >= x0 && s < x1) m |= (PX == 1 ? 0x11u : 0x1u) << c;
     }
     return m;
 }
+
+// a record's strip word beside the strip bits: its pairs need the cap of alpha and the power test
+constexpr uint32_t kNotPlain = 0x80000000u;
 
 // How a batch's records reach shared memory.
 constexpr int kGatherCpAsync = 0;  // every thread copies its record with 16-byte cp.async
 constexpr int kGatherTma = 1;      // one warp gathers four records per cp.async.bulk.tensor tile::gather4
 
-// The staging area of a batch (double-buffered). cp.async: full 3 x 16 B, p32 2 x 16 B, p24
-// 3 x 8 B per record (as uint2 rows of N in the first half of the area). TMA: quads of four
+// The staging area of a batch. cp.async: full 3 x 16 B, p32 2 x 16 B, p24 3 x 8 B per record (as uint2
+// rows of N in the first half of the area); a thread copies and reads its own record only, so one
+// buffer serves. TMA (double-buffered, one warp copies for all): quads of four
 // 48-byte records as gather4 writes them, each quad in a 256-byte slot so that every
 // destination is 128-byte aligned; one mbarrier per buffer and its completed uses (the phase).
 template <int N, int GATHER>
 struct StageArea {
-    float4 raw[2][3][N];
+    float4 raw[3][N];
 };
 template <int N>
 struct StageArea<N, kGatherTma> {
@@ -148,11 +176,13 @@ struct StageArea<N, kGatherTma> {
 template <int N, int GATHER = kGatherCpAsync>
 struct RenderShared {
     StageArea<N, GATHER> st;
-    float4 power0[N];     // qa, qb, qc, d of the expanded power (powerAt)
-    float4 power1[N];     // e, f, the sign-test bound, -
+    // (slot N of the prepared arrays: a record no pixel takes, which fills up a hit list's last group)
+    float4 power0[N + 1]; // qa, qb, qc, d of the expanded power (powerAt)
+    float4 power1[N + 1]; // e, f, the sign-test bound, -
+    float4 color[N + 1];  // r, g, b, -
     uint32_t strips[N];   // the warp strips the cutoff ellipse meets (stripMask)
-    float4 color[N];      // r, g, b, -
-    uint32_t hits[N / 32][32];  // per warp: the records of its current 32 that meet its strip, in list order
+    // per warp: the records of its current 32 that meet its strip, in list order (and the filling)
+    alignas(16) uint32_t hits[N / 32][32 + kHitGroup];
     uint32_t tile;        // persistent schedule: the block's current tile
 };
 
@@ -167,6 +197,24 @@ struct RenderShared {
 // must not drop the splat there).
 __device__ __forceinline__ float powerAt(const float4& u, const float4& w, float X, float Y) {
     return fmaf(X, fmaf(u.x, X, fmaf(u.y, Y, u.w)), fmaf(Y, fmaf(u.z, Y, w.x), w.y));
+}
+
+// U entries of a hit list
+template <uint32_t U>
+__device__ __forceinline__ void loadHits(const uint32_t* hits, uint32_t (&q)[U]) {
+    if constexpr (U == 4) {
+        const uint4 v = *reinterpret_cast<const uint4*>(hits);
+        q[0] = v.x;
+        q[1] = v.y;
+        q[2] = v.z;
+        q[3] = v.w;
+    } else if constexpr (U == 2) {
+        const uint2 v = *reinterpret_cast<const uint2*>(hits);
+        q[0] = v.x;
+        q[1] = v.y;
+    } else {
+        q[0] = hits[0];
+    }
 }
 
 __device__ __forceinline__ uint32_t smemAddr(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
@@ -198,6 +246,29 @@ __device__ __forceinline__ void mbarWaitBounded(uint64_t* bar, uint32_t parity, 
             return;
         }
     }
+}
+
+// INRIA's test-before-accept rule for one (pixel, splat) pair: nothing below alpha 1/255; a pair
+// that would leave less than minT of the transmittance T ends the pixel (minT becomes infinite, so
+// that no later pair is blended); any other is blended. One comparison yields both predicates.
+__device__ __forceinline__ void blendPair(float alpha, const float4& col, float& T, float& c0, float& c1, float& c2,
+                                          float& minT) {
+    asm("{\n"
+        " .reg .pred met, ends, blends;\n"
+        " .reg .f32 t, w;\n"
+        " setp.geu.f32 met, %5, 0f3B808081;\n"  // 1/255
+        " sub.f32 t, 0f3F800000, %5;\n"
+        " mul.f32 t, %0, t;\n"
+        " setp.lt.and.f32 ends|blends, t, %4, met;\n"
+        " @ends mov.f32 %4, 0f7F800000;\n"
+        " @blends mul.f32 w, %5, %0;\n"
+        " @blends fma.rn.f32 %1, %6, w, %1;\n"
+        " @blends fma.rn.f32 %2, %7, w, %2;\n"
+        " @blends fma.rn.f32 %3, %8, w, %3;\n"
+        " @blends mov.f32 %0, t;\n"
+        "}"
+        : "+f"(T), "+f"(c0), "+f"(c1), "+f"(c2), "+f"(minT)
+        : "f"(alpha), "f"(col.x), "f"(col.y), "f"(col.z));
 }
 
 // The view holding frame tile t: the last view whose tileBase <= t (views are in tile order).
@@ -308,10 +379,9 @@ __device__ __forceinline__ void windowPush(SortWindow<CAP>& q, uint32_t K, float
 // layout's kernel carries only its own gather and decode (a runtime switch measured 8 % slower).
 // CAP: 0, or the StopThePop window's register capacity; `ray` is then the shared area of the
 // gathered ray-depth parameters (3 x 16 B per entry, double-buffered).
-// TILE: the tile's code, 16 (INRIA's 16 x 16 tiles), 8 (8 x 8) or 32 (32 x 8); one thread per pixel, batches of
-// a tile's pixel count
-// entries, and each warp owns an 8 x 4 pixel block of the tile (its strip: a squarer footprint
-// meets fewer ellipses than a 16 x 2 row pair).
+// TILE: the tile's code, 16 (INRIA's 16 x 16 tiles), 8 (8 x 8) or 32 (32 x 8); one or two pixels a
+// thread (pixelsPerThread), batches of one entry a thread, and each warp owns an 8 x 4 or 8 x 8 pixel
+// block of the tile (its strip: a squarer footprint meets fewer ellipses than a 16 x 2 row pair).
 // STATS: the instrumented build (TileSettings::stats, tile_render.comp's GSR_TILE_STATS): the
 // kTileStatCount words of the tile (list length, fetched, evaluated, blended, terminated, lane
 // slots, max depth, pixels) and the frame's count of the pairs this kernel tested. "Evaluated"
@@ -321,12 +391,17 @@ __device__ __forceinline__ void windowPush(SortWindow<CAP>& q, uint32_t K, float
 // GATHER: how the batch reaches shared memory (kGatherCpAsync or kGatherTma; TMA only with the
 // full records, no window and no statistics); map = the tensor map of the record array (TMA).
 template <int MODE, int CAP, int TILE, bool STATS, int GATHER>
-__device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<tilePixels(TILE), GATHER>& sm,
-                                           float4 (*ray)[3][tilePixels(TILE)], uint32_t tile, const CUtensorMap* map) {
+__device__ __forceinline__ void renderTile(const RenderArgs& a,
+                                           RenderShared<tileThreads(CAP, TILE, STATS), GATHER>& sm,
+                                           float4 (*ray)[3][tileThreads(CAP, TILE, STATS)], uint32_t tile,
+                                           const CUtensorMap* map) {
     static_assert(GATHER == kGatherCpAsync || (MODE == kRenderSplatFull && CAP == 0 && !STATS), "the TMA gather");
     constexpr uint32_t kTW = tileW(TILE), kTH = tileH(TILE);
-    constexpr uint32_t kThreads = kTW * kTH, kStripW = 8, kRows = 4, kStripsX = kTW / kStripW;
-    static_assert(kThreads <= kRenderThreads && kStripW * kRows == 32 && kTW % kStripW == 0 && kTH % kRows == 0,
+    constexpr int PX = pixelsPerThread(CAP, TILE, STATS);
+    constexpr uint32_t kThreads = tileThreads(CAP, TILE, STATS), kStripW = 8, kRows = 4 * PX, kStripsX = kTW / kStripW;
+    constexpr uint32_t U = CAP == 0 && !STATS ? kHitGroup : 1;  // hits of a warp whose alphas are computed together
+    constexpr uint32_t kLanesX = kStripW / PX;  // lanes along a strip row, PX neighbouring pixels each
+    static_assert(kThreads <= kRenderThreads && kThreads * PX == kTW * kTH && kTW % kStripW == 0 && kTH % kRows == 0,
                   "tile shape");
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t sx = (warp % kStripsX) * kStripW, sy = (warp / kStripsX) * kRows;
@@ -334,8 +409,11 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
     const DevView vw = a.views[view];
     const uint32_t local = tile - vw.tileBase;
     const uint32_t tx = local % vw.tilesX, ty = local / vw.tilesX;
-    const uint32_t px = tx * kTW + sx + (lane % kStripW), py = ty * kTH + sy + (lane / kStripW);
-    const bool inside = px < vw.width && py < vw.height;
+    // the thread's pixels: (px, py) and for PX = 2 its right neighbour
+    const uint32_t px = tx * kTW + sx + PX * (lane % kLanesX), py = ty * kTH + sy + (lane / kLanesX);
+    bool inside[PX];
+#pragma unroll
+    for (int k = 0; k < PX; ++k) inside[k] = px + k < vw.width && py < vw.height;
     uint2 range = reinterpret_cast<const uint2*>(a.ranges)[tile];
     // a frame whose look-back gave up (GSR_CONTROL_TIMEOUT) has meaningless ranges: every index
     // read below stays inside the list and the scene all the same
@@ -356,8 +434,17 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
     // -8..7: the expansion's terms stay small against the power it sums to)
     const float X = float(int(px) - int((tx * kTW) & ~31u) - 16), Y = float(int(py) - int((ty * kTH) & ~15u) - 8);
     // this warp's pixel strip
-    float T = 1.0f, c0 = 0.0f, c1 = 0.0f, c2 = 0.0f;
-    bool done = !inside;
+    float T[PX], c0[PX], c1[PX], c2[PX];
+    bool done[PX];
+    float minT[PX];  // the least transmittance a blend may leave; infinite once the pixel is done
+#pragma unroll
+    for (int k = 0; k < PX; ++k) {
+        T[k] = 1.0f;
+        c0[k] = c1[k] = c2[k] = 0.0f;
+        done[k] = !inside[k];
+        minT[k] = inside[k] ? kMinTransmittance : __int_as_float(0x7f800000);
+    }
+    auto allDone = [&]() { return PX == 1 ? done[0] : (done[0] && done[PX - 1]); };
 
     // TMA: the buffers' mbarrier phases, the same in every thread (each thread counts the uses)
     uint32_t phase0 = 0, phase1 = 0;
@@ -365,6 +452,12 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
         phase0 = sm.st.uses[0];
         phase1 = sm.st.uses[1];
     }
+    // cp.async: the gaussian of the next batch's entry, loaded a batch ahead of the copies that need it
+    uint32_t index = 0;
+    auto fetchIndex = [&](uint32_t start) {
+        const uint32_t j = start + tid;
+        if (j < range.y) index = packed ? uint32_t(__ldg(&packedKeys[j]) & indexMask) : __ldg(&values[j]);
+    };
     auto issue = [&](uint32_t start, int buf) {
         if constexpr (GATHER == kGatherTma) {
             // warp 0 reads the batch's gaussian indices and gathers the records four at a time
@@ -391,25 +484,24 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
                 tmaGather4(&sm.st.quad[buf][q][0], map, row, &sm.st.bar[buf]);
             }
         } else {
-            const uint32_t j = start + tid;
-            if (j < range.y) {
-                uint32_t g = packed ? uint32_t(__ldg(&packedKeys[j]) & indexMask) : __ldg(&values[j]);
+            if (start + tid < range.y) {
+                uint32_t g = index;
                 if (g >= a.count) {
                     atomicOr(&a.ctl->c.status, uint32_t(GSR_CONTROL_BOUNDS));
                     g = 0;
                 }
                 if constexpr (mode == kRenderSplatFull) {
                     const float4* rec = records + size_t(g) * 3;
-                    cpAsync16(&sm.st.raw[buf][0][tid], rec);
-                    cpAsync16(&sm.st.raw[buf][1][tid], rec + 1);
-                    cpAsync16(&sm.st.raw[buf][2][tid], rec + 2);
+                    cpAsync16(&sm.st.raw[0][tid], rec);
+                    cpAsync16(&sm.st.raw[1][tid], rec + 1);
+                    cpAsync16(&sm.st.raw[2][tid], rec + 2);
                 } else if constexpr (mode == kRenderSplatP32) {
                     const uint4* rec = records32 + size_t(g) * 2;
-                    cpAsync16(&sm.st.raw[buf][0][tid], rec);
-                    cpAsync16(&sm.st.raw[buf][1][tid], rec + 1);
+                    cpAsync16(&sm.st.raw[0][tid], rec);
+                    cpAsync16(&sm.st.raw[1][tid], rec + 1);
                 } else {  // 24-byte records start on 8-byte boundaries
                     const uint2* rec = records24 + size_t(g) * 3;
-                    uint2* dst = reinterpret_cast<uint2*>(&sm.st.raw[buf][0][0]);
+                    uint2* dst = reinterpret_cast<uint2*>(&sm.st.raw[0][0]);
                     cpAsync8(&dst[tid], rec);
                     cpAsync8(&dst[kThreads + tid], rec + 1);
                     cpAsync8(&dst[2 * kThreads + tid], rec + 2);
@@ -422,6 +514,7 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
                 }
             }
             cpAsyncCommit();
+            fetchIndex(start + kThreads);
         }
     };
     // TMA: every thread waits for the buffer's gathers (bounded) and counts the use
@@ -451,15 +544,19 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
     // preparation. Every batch issued is waited for at the top of the next iteration, which
     // always runs, so none is in flight after the loop.
     int buf = 0;
-    if (range.x < range.y) issue(range.x, 0);
+    if (range.x < range.y) {
+        if constexpr (GATHER == kGatherCpAsync) fetchIndex(range.x);
+        issue(range.x, 0);
+    }
     for (uint32_t start = range.x; start < range.y; start += kThreads, buf ^= 1) {
         if constexpr (GATHER == kGatherTma) waitTma(buf);
         else cpAsyncWait<0>();
-        if (__syncthreads_count(done) == int(kThreads)) break;
+        if (__syncthreads_count(allDone()) == int(kThreads)) break;
         if constexpr (STATS) stFetched += range.y - start < kThreads ? range.y - start : kThreads;
-        // the next batch is gathered while this one is prepared and blended
+        // the next batch is gathered while this one is blended (TMA: prepared and blended)
         const uint32_t next = start + kThreads;
-        if (next < range.y) issue(next, buf ^ 1);
+        if constexpr (GATHER == kGatherTma)
+            if (next < range.y) issue(next, buf ^ 1);
         if (start + tid < range.y) {
             float2 r0;  // cx, cy
             float A, B, C, o;
@@ -473,9 +570,9 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
                     w1 = rec[1];
                     r2 = rec[2];
                 } else {
-                    w0 = sm.st.raw[buf][0][tid];  // cx, cy, depth, cull
-                    w1 = sm.st.raw[buf][1][tid];  // A, B, C, opacity
-                    r2 = sm.st.raw[buf][2][tid];  // r, g, b, radius
+                    w0 = sm.st.raw[0][tid];  // cx, cy, depth, cull
+                    w1 = sm.st.raw[1][tid];  // A, B, C, opacity
+                    r2 = sm.st.raw[2][tid];  // r, g, b, radius
                 }
                 r0 = make_float2(w0.x, w0.y);
                 A = w1.x;
@@ -484,8 +581,8 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
                 o = w1.w;
                 radius = r2.w;
             } else if constexpr (mode == kRenderSplatP32) {
-                const float4 w0 = sm.st.raw[buf][0][tid];  // cx, cy, A, B
-                const float4 w1 = sm.st.raw[buf][1][tid];  // C, opacity, h(r, g), h(b) | radius
+                const float4 w0 = sm.st.raw[0][tid];  // cx, cy, A, B
+                const float4 w1 = sm.st.raw[1][tid];  // C, opacity, h(r, g), h(b) | radius
                 r0 = make_float2(w0.x, w0.y);
                 A = w0.z;
                 B = w0.w;
@@ -495,7 +592,7 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
                 r2 = make_float4(halfLoF(rg), halfHiF(rg), halfLoF(bw), 0.0f);
                 radius = float(bw >> 16);
             } else {
-                const uint2* w = reinterpret_cast<const uint2*>(&sm.st.raw[buf][0][0]);
+                const uint2* w = reinterpret_cast<const uint2*>(&sm.st.raw[0][0]);
                 const uint2 w0 = w[tid], w1 = w[kThreads + tid], w2 = w[2 * kThreads + tid];
                 r0 = make_float2(__uint_as_float(w0.x), __uint_as_float(w0.y));
                 p24DecodeConic(w1.x, w1.y, A, B, C, o);
@@ -514,14 +611,13 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
                 const float rho = fabsf(B) * rsqrtf(A * C);
                 const float K = 2.0f / fmaxf(1.0f - rho, 1e-30f);
                 const float t = qmax + (2e-3f + 4e-5f * K) * fmaxf(qmax, 1.0f) + 4e-3f;
-                if (t < 1e30f) strips = stripMask<TILE>(r0.x, r0.y, A, B, C, D, t, float(tx * kTW), float(ty * kTH));
+                if (t < 1e30f) strips = stripMask<TILE, PX>(r0.x, r0.y, A, B, C, D, t, float(tx * kTW), float(ty * kTH));
             }
             // 32 x 8 tiles: a bin's 32 columns can reach 16 px past the splat's 16-px rectangle,
             // which bounds the splat's pixels wherever the coverage used it (rect and tight
             // bounds, and cutoff-only bounds for a splat without an ellipse)
             if constexpr (TILE == 32)
-                if (a.bounds != kBoundsCutoff || !ellipse) strips &= rectStrips32(r0.x, radius, tx * kTW);
-            sm.strips[tid] = strips;
+                if (a.bounds != kBoundsCutoff || !ellipse) strips &= rectStrips32<PX>(r0.x, radius, tx * kTW);
             // the expanded power about the cell origin (powerAt); only a record with strips is
             // visited, so its opacity is at least 1/255 and log2(o) finite
             const float qa = -0.5f * kLog2e * A, qb = -kLog2e * B, qc = -0.5f * kLog2e * C;
@@ -529,10 +625,23 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
             const float cx = r0.x - (float(px) - X), cy = r0.y - (float(py) - Y);  // the cell centre: exact
             const float d = -fmaf(2.0f * qa, cx, qb * cy), e = -fmaf(2.0f * qc, cy, qb * cx);
             const float f = fmaf(cx, fmaf(qa, cx, qb * cy), fmaf(cy, qc * cy, lg));
+            if constexpr (CAP == 0 && !STATS) {
+                // PLAIN records need neither the cap of alpha at 0.99 nor the power test: an ellipse
+                // whose computed exponent stays below log2(0.99) at every pixel of the cell. The
+                // exact one is at most lg; the sum's and the terms' roundings are below 2^-19 of
+                // the terms' magnitudes (a dozen roundings of 2^-24 each).
+                const float X0 = 17.0f + fabsf(cx), Y0 = 9.0f + fabsf(cy);
+                const float size = -qa * X0 * X0 + fabsf(qb) * X0 * Y0 - qc * Y0 * Y0 + fabsf(lg);
+                if (!(ellipse && fmaf(size, 1.91e-6f, lg) < -0.015f)) strips |= kNotPlain;  // log2(0.99) = -0.0145
+            }
+            sm.strips[tid] = strips;
             sm.power0[tid] = make_float4(qa, qb, qc, d);
             sm.power1[tid] = make_float4(e, f, ellipse ? __int_as_float(0x7f800000) : lg, 0.0f);
             sm.color[tid] = r2;
         }
+        // (each thread has read its own records: its next ones may be copied over them)
+        if constexpr (GATHER == kGatherCpAsync)
+            if (next < range.y) issue(next, buf ^ 1);
         __syncthreads();
         const uint32_t n = range.y - start < kThreads ? range.y - start : kThreads;
         // the warp takes 32 records at a time, one per lane, lists those that meet its strip in
@@ -540,50 +649,91 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
         // list: a load a record instead of finding and clearing the next set bit of the ballot
         uint32_t* hits = sm.hits[warp];
         const uint32_t below = (1u << lane) - 1u;
-        for (uint32_t q0 = 0; q0 < n && !__all_sync(0xffffffffu, done); q0 += 32) {
+        for (uint32_t q0 = 0; q0 < n && !__all_sync(0xffffffffu, allDone()); q0 += 32) {
             const uint32_t ql = q0 + lane;
-            const bool hit = ql < n && ((sm.strips[ql] >> warp) & 1u) != 0u;
+            const uint32_t strips = ql < n ? sm.strips[ql] : 0u;
+            const bool hit = ((strips >> warp) & 1u) != 0u;
             const uint32_t m = __ballot_sync(0xffffffffu, hit);
             if (hit) hits[__popc(m & below)] = ql;
-            __syncwarp();
             const uint32_t listed = uint32_t(__popc(m));
-            for (uint32_t h = 0; h < listed; ++h) {
-                const uint32_t q = hits[h];
-                if constexpr (STATS) {
-                    ++stIters;
-                    stTested += done ? 0u : 1u;
-                }
-                const float4 pw0 = sm.power0[q], pw1 = sm.power1[q];
-                const float p = powerAt(pw0, pw1, X, Y);
-                const float alpha = fminf(kMaxAlpha, fastExp2(p));
-                // skipped: a finished pixel, power > 0, alpha below 1/255 (one predicate)
-                if (done || p > pw1.z || alpha < (1.0f / 255.0f)) continue;
-                if constexpr (CAP > 0) {
-                    // the depth of the gaussian's maximum along the pixel ray: (v . b) / (v^T P v)
-                    const float4 pa = ray[buf][0][q], pb = ray[buf][1][q];
-                    const float pc = ray[buf][2][q].x;
-                    const float vPv = pa.x * vx * vx + 2.0f * pa.y * vx * vy + 2.0f * pa.z * vx + pa.w * vy * vy +
-                                      2.0f * pb.x * vy + pb.y;
-                    const float vb = pb.z * vx + pb.w * vy + pc;
-                    windowPush(window, K, vb / vPv, alpha, sm.color[q], T, c0, c1, c2, done);
-                    continue;
-                }
-                const float testT = T * (1.0f - alpha);
-                if (testT < kMinTransmittance) {
-                    done = true;
-                    if constexpr (STATS) {
-                        stTerm = true;
-                        stEval = start + q - range.x + 1u;  // the entries visited, the terminating one included
+            if (U > 1 && lane < U) hits[listed + lane] = kThreads;  // fills the last group
+            __syncwarp();
+            if constexpr (CAP == 0 && !STATS) {
+                // PLAIN: every listed record's alpha is below the cap and its power never positive
+                auto walk = [&](auto plain) {
+                    for (uint32_t h = 0; h < listed; h += U) {
+                        uint32_t q[U];
+                        loadHits<U>(hits + h, q);
+#pragma unroll
+                        for (uint32_t u = 0; u < U; ++u) {
+                            const float4 pw0 = sm.power0[q[u]];
+                            float alpha[PX];
+                            if constexpr (decltype(plain)::value) {
+                                const float2 pw1 = *reinterpret_cast<const float2*>(&sm.power1[q[u]]);
+                                const float rowLin = fmaf(pw0.y, Y, pw0.w), rowSum = fmaf(Y, fmaf(pw0.z, Y, pw1.x), pw1.y);
+#pragma unroll
+                                for (int k = 0; k < PX; ++k) {
+                                    const float x = X + float(k);
+                                    alpha[k] = fastExp2(fmaf(x, fmaf(pw0.x, x, rowLin), rowSum));
+                                }
+                            } else {
+                                const float4 pw1 = sm.power1[q[u]];
+                                const float rowLin = fmaf(pw0.y, Y, pw0.w), rowSum = fmaf(Y, fmaf(pw0.z, Y, pw1.x), pw1.y);
+#pragma unroll
+                                for (int k = 0; k < PX; ++k) {
+                                    const float x = X + float(k), p = fmaf(x, fmaf(pw0.x, x, rowLin), rowSum);
+                                    alpha[k] = p > pw1.z ? 0.0f : fminf(kMaxAlpha, fastExp2(p));
+                                }
+                            }
+                            const float4 col = sm.color[q[u]];
+#pragma unroll
+                            for (int k = 0; k < PX; ++k) blendPair(alpha[k], col, T[k], c0[k], c1[k], c2[k], minT[k]);
+                        }
                     }
-                    continue;
+                };
+                if (__any_sync(0xffffffffu, hit && (strips & kNotPlain))) walk(std::false_type{});
+                else walk(std::true_type{});
+#pragma unroll
+                for (int k = 0; k < PX; ++k) done[k] = minT[k] > 1.0f;
+            } else {
+                for (uint32_t h = 0; h < listed; ++h) {
+                    const uint32_t q = hits[h];
+                    if constexpr (STATS) {
+                        ++stIters;
+                        stTested += done[0] ? 0u : 1u;
+                    }
+                    const float4 pw0 = sm.power0[q], pw1 = sm.power1[q];
+                    const float p = powerAt(pw0, pw1, X, Y);
+                    const float alpha = fminf(kMaxAlpha, fastExp2(p));
+                    // skipped: a finished pixel, power > 0, alpha below 1/255 (one predicate)
+                    if (done[0] || p > pw1.z || alpha < (1.0f / 255.0f)) continue;
+                    if constexpr (CAP > 0) {
+                        // the depth of the gaussian's maximum along the pixel ray: (v . b) / (v^T P v)
+                        const float4 pa = ray[buf][0][q], pb = ray[buf][1][q];
+                        const float pc = ray[buf][2][q].x;
+                        const float vPv = pa.x * vx * vx + 2.0f * pa.y * vx * vy + 2.0f * pa.z * vx + pa.w * vy * vy +
+                                          2.0f * pb.x * vy + pb.y;
+                        const float vb = pb.z * vx + pb.w * vy + pc;
+                        windowPush(window, K, vb / vPv, alpha, sm.color[q], T[0], c0[0], c1[0], c2[0], done[0]);
+                        continue;
+                    }
+                    const float testT = T[0] * (1.0f - alpha);
+                    if (testT < kMinTransmittance) {
+                        done[0] = true;
+                        if constexpr (STATS) {
+                            stTerm = true;
+                            stEval = start + q - range.x + 1u;  // the entries visited, the terminating one included
+                        }
+                        continue;
+                    }
+                    const float4 col = sm.color[q];
+                    const float w = alpha * T[0];
+                    c0[0] += col.x * w;
+                    c1[0] += col.y * w;
+                    c2[0] += col.z * w;
+                    T[0] = testT;
+                    if constexpr (STATS) ++stBlend;
                 }
-                const float4 col = sm.color[q];
-                const float w = alpha * T;
-                c0 += col.x * w;
-                c1 += col.y * w;
-                c2 += col.z * w;
-                T = testT;
-                if constexpr (STATS) ++stBlend;
             }
             __syncwarp();  // every lane has read the list before the next group writes it
         }
@@ -591,7 +741,8 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
     if constexpr (CAP > 0) {  // the end of the list: what waits is blended, nearest first
 #pragma unroll
         for (int i = 0; i < CAP; ++i)
-            if (!done && uint32_t(i) < window.count) blendOver(window.al[i], window.r[i], window.g[i], window.b[i], T, c0, c1, c2, done);
+            if (!done[0] && uint32_t(i) < window.count)
+                blendOver(window.al[i], window.r[i], window.g[i], window.b[i], T[0], c0[0], c1[0], c2[0], done[0]);
     }
     if constexpr (GATHER == kGatherTma) {
         // no batch is in flight here (see the loop); the phases are kept for the next tile
@@ -604,12 +755,12 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
         cpAsyncWait<0>();
     }
     if constexpr (STATS) {
-        if (!stTerm) stEval = inside ? range.y - range.x : 0u;
+        if (!stTerm) stEval = inside[0] ? range.y - range.x : 0u;
         __shared__ uint32_t sStat[kTileStatWords];
         if (tid < kTileStatWords) sStat[tid] = 0u;
         __syncthreads();
         const uint32_t eSum = __reduce_add_sync(0xffffffffu, stEval), bSum = __reduce_add_sync(0xffffffffu, stBlend);
-        const uint32_t tSum = __popc(__ballot_sync(0xffffffffu, stTerm)), pSum = __popc(__ballot_sync(0xffffffffu, inside));
+        const uint32_t tSum = __popc(__ballot_sync(0xffffffffu, stTerm)), pSum = __popc(__ballot_sync(0xffffffffu, inside[0]));
         const uint32_t eMax = __reduce_max_sync(0xffffffffu, stEval), tested = __reduce_add_sync(0xffffffffu, stTested);
         if (lane == 0) {
             atomicAdd(&sStat[kTileStatEvaluated], eSum);
@@ -628,28 +779,31 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<til
         __syncthreads();
         if (tid < kTileStatWords) a.tileStats[size_t(tile) * kTileStatWords + tid] = sStat[tid];
     }
-    if (!inside) return;
-    const size_t p = vw.pixelBase + size_t(py) * vw.width + px;
-    if (a.imageFormat == 0) {
-        reinterpret_cast<float4*>(a.image)[p] = make_float4(c0, c1, c2, 1.0f - T);
-    } else if (a.imageFormat == 1) {
-        reinterpret_cast<uint2*>(a.image)[p] = make_uint2(packHalf2(c0, c1), packHalf2(c2, 1.0f - T));
-    } else {
-        const float v[4] = {c0, c1, c2, 1.0f - T};
-        uint32_t w = 0;
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {
-            const float cl = v[ch] < 0.0f ? 0.0f : (v[ch] > 1.0f ? 1.0f : v[ch]);
-            w |= uint32_t(roundf(cl * 255.0f)) << (8 * ch);
+    for (int k = 0; k < PX; ++k) {
+        if (!inside[k]) continue;
+        const size_t p = vw.pixelBase + size_t(py) * vw.width + px + k;
+        if (a.imageFormat == 0) {
+            reinterpret_cast<float4*>(a.image)[p] = make_float4(c0[k], c1[k], c2[k], 1.0f - T[k]);
+        } else if (a.imageFormat == 1) {
+            reinterpret_cast<uint2*>(a.image)[p] = make_uint2(packHalf2(c0[k], c1[k]), packHalf2(c2[k], 1.0f - T[k]));
+        } else {
+            const float v[4] = {c0[k], c1[k], c2[k], 1.0f - T[k]};
+            uint32_t w = 0;
+#pragma unroll
+            for (int ch = 0; ch < 4; ++ch) {
+                const float cl = v[ch] < 0.0f ? 0.0f : (v[ch] > 1.0f ? 1.0f : v[ch]);
+                w |= uint32_t(roundf(cl * 255.0f)) << (8 * ch);
+            }
+            reinterpret_cast<uint32_t*>(a.image)[p] = w;
         }
-        reinterpret_cast<uint32_t*>(a.image)[p] = w;
-    }
-    if (a.rgb8) {
-        const float v[3] = {c0, c1, c2};
+        if (a.rgb8) {
+            const float v[3] = {c0[k], c1[k], c2[k]};
 #pragma unroll
-        for (int ch = 0; ch < 3; ++ch) {
-            const float cl = v[ch] < 0.0f ? 0.0f : (v[ch] > 1.0f ? 1.0f : v[ch]);
-            a.rgb8[p * 3 + ch] = uint8_t(roundf(cl * 255.0f));  // lround(clamp(v, 0, 1) * 255), image_io.cpp:55-56
+            for (int ch = 0; ch < 3; ++ch) {
+                const float cl = v[ch] < 0.0f ? 0.0f : (v[ch] > 1.0f ? 1.0f : v[ch]);
+                a.rgb8[p * 3 + ch] = uint8_t(roundf(cl * 255.0f));  // lround(clamp(v, 0, 1) * 255), image_io.cpp:55-56
+            }
         }
     }
 }
@@ -668,6 +822,11 @@ __device__ __forceinline__ float4 (*rayArea(unsigned char* smem))[3][N] {
 // TMA: the buffers' mbarriers, initialized once per block (their phases then run across tiles)
 template <int N, int GATHER>
 __device__ __forceinline__ void initStage(RenderShared<N, GATHER>& sm) {
+    if (threadIdx.x == 0) {  // read after the first batch's barriers
+        sm.power0[N] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        sm.power1[N] = make_float4(0.0f, __int_as_float(0xff800000), __int_as_float(0x7f800000), 0.0f);  // 2^-inf = 0
+        sm.color[N] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
     if constexpr (GATHER == kGatherTma) {
         if (threadIdx.x == 0) {
             for (int b = 0; b < 2; ++b) {
@@ -680,32 +839,32 @@ __device__ __forceinline__ void initStage(RenderShared<N, GATHER>& sm) {
     }
 }
 
-// Without the window: five 256-thread blocks (or the same threads in 8-px tiles) per SM, 48
-// registers a thread (the strip masks would take 61, four blocks, 5 % slower).
 template <int MODE, int CAP, int TILE, bool STATS, int GATHER>
-__global__ void __launch_bounds__(tilePixels(TILE), CAP == 0 ? 5 * 256 / (tilePixels(TILE)) : 1)
+__global__ void __launch_bounds__(tileThreads(CAP, TILE, STATS), CAP == 0 ? kResidentThreads / tileThreads(CAP, TILE, STATS) : 1)
     renderKernel(const __grid_constant__ RenderArgs a, const __grid_constant__ CUtensorMap map) {
     extern __shared__ __align__(128) unsigned char smemRaw[];
-    RenderShared<tilePixels(TILE), GATHER>& sm = *reinterpret_cast<RenderShared<tilePixels(TILE), GATHER>*>(smemRaw);
+    constexpr int N = tileThreads(CAP, TILE, STATS);
+    RenderShared<N, GATHER>& sm = *reinterpret_cast<RenderShared<N, GATHER>*>(smemRaw);
     initStage(sm);
-    renderTile<MODE, CAP, TILE, STATS, GATHER>(a, sm, CAP > 0 ? rayArea<tilePixels(TILE), GATHER>(smemRaw) : nullptr,
+    renderTile<MODE, CAP, TILE, STATS, GATHER>(a, sm, CAP > 0 ? rayArea<N, GATHER>(smemRaw) : nullptr,
                                                blockIdx.x + a.tileOffset, &map);
 }
 
 // Persistent schedule: each block takes tiles from the frame's queue counter (reset by frame
 // begin) until the counter passes the last tile.
 template <int MODE, int CAP, int TILE, bool STATS, int GATHER>
-__global__ void __launch_bounds__(tilePixels(TILE), CAP == 0 ? 5 * 256 / (tilePixels(TILE)) : 1)
+__global__ void __launch_bounds__(tileThreads(CAP, TILE, STATS), CAP == 0 ? kResidentThreads / tileThreads(CAP, TILE, STATS) : 1)
     renderPersistentKernel(const __grid_constant__ RenderArgs a, const __grid_constant__ CUtensorMap map) {
     extern __shared__ __align__(128) unsigned char smemRaw[];
-    RenderShared<tilePixels(TILE), GATHER>& sm = *reinterpret_cast<RenderShared<tilePixels(TILE), GATHER>*>(smemRaw);
+    constexpr int N = tileThreads(CAP, TILE, STATS);
+    RenderShared<N, GATHER>& sm = *reinterpret_cast<RenderShared<N, GATHER>*>(smemRaw);
     initStage(sm);
     for (;;) {
         if (threadIdx.x == 0) sm.tile = atomicAdd(&a.ctl->tickets[kRenderQueueTicket], 1u);
         __syncthreads();
         const uint32_t tile = sm.tile;
         if (tile >= a.totalTiles) break;
-        renderTile<MODE, CAP, TILE, STATS, GATHER>(a, sm, CAP > 0 ? rayArea<tilePixels(TILE), GATHER>(smemRaw) : nullptr,
+        renderTile<MODE, CAP, TILE, STATS, GATHER>(a, sm, CAP > 0 ? rayArea<N, GATHER>(smemRaw) : nullptr,
                                                    tile, &map);
         __syncthreads();  // every thread has read sm.tile and left the tile's shared buffers
     }
@@ -713,8 +872,8 @@ __global__ void __launch_bounds__(tilePixels(TILE), CAP == 0 ? 5 * 256 / (tilePi
 
 template <int MODE, int CAP, int TILE, bool STATS = false, int GATHER = kGatherCpAsync>
 cudaError_t launchRenderMode(const RenderArgs& a, cudaStream_t s) {
-    constexpr size_t smem = renderSmemBytes<CAP, tilePixels(TILE), GATHER>();
-    constexpr uint32_t threads = tilePixels(TILE);
+    constexpr uint32_t threads = tileThreads(CAP, TILE, STATS);
+    constexpr size_t smem = renderSmemBytes<CAP, tileThreads(CAP, TILE, STATS), GATHER>();
     static std::atomic<bool> configuredOn[64] = {};
     std::atomic<bool>& configured = perDevice(configuredOn);
     if (!configured) {
