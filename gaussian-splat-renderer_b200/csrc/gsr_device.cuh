@@ -36,11 +36,13 @@ __device__ __forceinline__ uint64_t ldRelaxed(const uint64_t* p) {
 __device__ __forceinline__ void stRelaxed(uint64_t* p, uint64_t v) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-__device__ __forceinline__ uint32_t ldAcquire32(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
+// First statement (beside the set-up of a block's own shared memory) of every kernel that a frame
+// launches with launchDependent: waits until the kernel before it has completed and its writes are
+// visible. Nothing another kernel of the frame writes is read before it, nor through the read-only
+// path (ld.global.nc). A kernel lets the next one be placed when it ends, not earlier: with
+// griddepcontrol.launch_dependents at its start the waiting blocks took the places of running ones
+// (8-view frame 3.39 -> 3.60 ms, 4K 2.16 -> 2.29 ms, small frames unchanged).
+__device__ __forceinline__ void gridWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Look-back status words: [63:34] epoch, [33:32] flag, [31:0] value.
 constexpr uint64_t kFlagAggregate = 1, kFlagInclusive = 2;

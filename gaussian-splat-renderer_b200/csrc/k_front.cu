@@ -313,7 +313,7 @@ __device__ __forceinline__ void learnedColour(const FrontArgs& a, LearnedShared&
     if (a.decoded) {  // decoded by the tensor-core pre-pass
         if (visible) {
             if (!latentIsFallback(__ldg(&a.latents[i]))) {
-                const float4 c = __ldg(&a.decoded[rec]);
+                const float4 c = __ldcg(&a.decoded[rec]);
                 s.r = c.x;
                 s.g = c.y;
                 s.b = c.z;
@@ -403,6 +403,7 @@ __global__ void __launch_bounds__(kFrontThreads, 4) preprocessKernel(const __gri
     __shared__ uint32_t sCull[kCullReasonCount];
     __shared__ uint32_t sDepthMin, sDepthMax;
     const uint32_t tid = threadIdx.x, lane = tid & 31;
+    gridWait();
     // the views vary fastest along the grid: the blocks of one gaussian range for every view run
     // side by side, so one of them reads the range's scene data from DRAM and the others from L2
     const uint32_t view = blockIdx.x % a.viewCount, i0 = blockIdx.x / a.viewCount * kFrontThreads;
@@ -526,6 +527,7 @@ __global__ void __launch_bounds__(kFrontThreads, 4) preprocessKernel(const __gri
 template <bool BINNING>
 __global__ void __launch_bounds__(kFrontThreads) duplicateKernel(const __grid_constant__ FrontArgs a) {
     __shared__ uint32_t sTileMax, sMismatch, sAny;
+    gridWait();
     const uint32_t tid = threadIdx.x;
     if (tid == 0) {
         sTileMax = 0;
@@ -701,6 +703,7 @@ __global__ void __launch_bounds__(kFrontThreads) duplicateKernel(const __grid_co
 __global__ void frameBeginKernel(DeviceControl* ctl, uint32_t count, uint32_t capacity, uint4* ranges,
                                  uint32_t rangeVec4s, SortPlan* plan, uint32_t forceTimeout, SortPlan* plan2,
                                  uint32_t* clear, uint32_t clearCount) {
+    gridWait();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     for (uint32_t j = g; j < rangeVec4s; j += gridDim.x * blockDim.x) ranges[j] = make_uint4(0, 0, 0, 0);
     for (uint32_t j = g; j < clearCount; j += gridDim.x * blockDim.x) clear[j] = 0;
@@ -807,6 +810,7 @@ template <int GEOM>
 __global__ void __launch_bounds__(kDecodeTcThreads) decodeColoursTcKernel(const __grid_constant__ FrontArgs a) {
     extern __shared__ __align__(128) unsigned char decodeRaw[];
     DecodeTcSmem& S = *reinterpret_cast<DecodeTcSmem*>(decodeRaw + ((128u - (tc::smem32(decodeRaw) & 127u)) & 127u));
+    gridWait();
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
     const DecoderWeights& W = *a.decoder;
     // the weights in the operand layout, the biases, the barrier and the tensor memory
@@ -969,7 +973,7 @@ void launchPreprocessT(const FrontArgs& a, dim3 blocks, cudaStream_t s) {
         configured = cudaFuncSetAttribute(preprocessKernel<GEOM, COLOR, LEARNED, EXTRAS>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, kShStageBytes) == cudaSuccess;
     }
-    preprocessKernel<GEOM, COLOR, LEARNED, EXTRAS><<<blocks, kFrontThreads, a.shStaged ? kShStageBytes : 0, s>>>(a);
+    launchDependent(preprocessKernel<GEOM, COLOR, LEARNED, EXTRAS>, blocks, kFrontThreads, a.shStaged ? kShStageBytes : 0, s, a);
 }
 template <int GEOM, int COLOR>
 void launchPreprocess(const FrontArgs& a, dim3 blocks, cudaStream_t s) {
@@ -1044,8 +1048,7 @@ cudaError_t launchFrontBinningEmit(const FrontArgs& a, cudaStream_t s) {
     cudaError_t e = launchScan(a.tileCounts, nullptr, a.offsets, &a.ctl->c.duplicates, records, kScanGatherSorted,
                                a.scanStatus, a.ctl, s, a.capacity, kWaitScan, &gather);
     if (e != cudaSuccess) return e;
-    duplicateKernel<true><<<(records + kFrontThreads - 1) / kFrontThreads, kFrontThreads, 0, s>>>(a);
-    return cudaGetLastError();
+    return launchDependent(duplicateKernel<true>, dim3((records + kFrontThreads - 1) / kFrontThreads), kFrontThreads, 0, s, a);
 }
 
 namespace {
@@ -1064,8 +1067,7 @@ cudaError_t launchDecodeTcT(const FrontArgs& a, cudaStream_t s) {
     }
     const uint32_t tiles = (a.count + 127u) / 128u * a.viewCount;
     const uint32_t blocks = tiles < uint32_t(grid) ? tiles : uint32_t(grid);
-    decodeColoursTcKernel<GEOM><<<blocks, kDecodeTcThreads, kDecodeTcSmem, s>>>(a);
-    return cudaGetLastError();
+    return launchDependent(decodeColoursTcKernel<GEOM>, dim3(blocks), kDecodeTcThreads, kDecodeTcSmem, s, a);
 }
 }  // namespace
 
@@ -1101,8 +1103,7 @@ cudaError_t launchFront(const FrontArgs& a, uint32_t geometry, uint32_t color, c
                    a.scanStatus, a.ctl, s, a.capacity, kWaitScan);
     if (e != cudaSuccess) return e;
     // 3) key emission
-    duplicateKernel<false><<<blocks, kFrontThreads, 0, s>>>(a);
-    return cudaGetLastError();
+    return launchDependent(duplicateKernel<false>, blocks, kFrontThreads, 0, s, a);
 }
 
 cudaError_t launchLogfTable(float* out, LogfFixups t, cudaStream_t s) {

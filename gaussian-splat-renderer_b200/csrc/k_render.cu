@@ -456,7 +456,7 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a,
     uint32_t index = 0;
     auto fetchIndex = [&](uint32_t start) {
         const uint32_t j = start + tid;
-        if (j < range.y) index = packed ? uint32_t(__ldg(&packedKeys[j]) & indexMask) : __ldg(&values[j]);
+        if (j < range.y) index = packed ? uint32_t(__ldcg(&packedKeys[j]) & indexMask) : __ldcg(&values[j]);
     };
     auto issue = [&](uint32_t start, int buf) {
         if constexpr (GATHER == kGatherTma) {
@@ -474,7 +474,7 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a,
                 for (uint32_t r = 0; r < 4; ++r) {
                     const uint32_t slot = 4u * q + r;
                     const uint32_t j = start + (slot < n ? slot : n - 1u);  // a short last quad repeats its last record
-                    uint32_t g = packed ? uint32_t(__ldg(&packedKeys[j]) & indexMask) : __ldg(&values[j]);
+                    uint32_t g = packed ? uint32_t(__ldcg(&packedKeys[j]) & indexMask) : __ldcg(&values[j]);
                     if (g >= a.count) {
                         atomicOr(&a.ctl->c.status, uint32_t(GSR_CONTROL_BOUNDS));
                         g = 0;
@@ -846,6 +846,7 @@ __global__ void __launch_bounds__(tileThreads(CAP, TILE, STATS), CAP == 0 ? kRes
     constexpr int N = tileThreads(CAP, TILE, STATS);
     RenderShared<N, GATHER>& sm = *reinterpret_cast<RenderShared<N, GATHER>*>(smemRaw);
     initStage(sm);
+    gridWait();
     renderTile<MODE, CAP, TILE, STATS, GATHER>(a, sm, CAP > 0 ? rayArea<N, GATHER>(smemRaw) : nullptr,
                                                blockIdx.x + a.tileOffset, &map);
 }
@@ -859,6 +860,7 @@ __global__ void __launch_bounds__(tileThreads(CAP, TILE, STATS), CAP == 0 ? kRes
     constexpr int N = tileThreads(CAP, TILE, STATS);
     RenderShared<N, GATHER>& sm = *reinterpret_cast<RenderShared<N, GATHER>*>(smemRaw);
     initStage(sm);
+    gridWait();
     for (;;) {
         if (threadIdx.x == 0) sm.tile = atomicAdd(&a.ctl->tickets[kRenderQueueTicket], 1u);
         __syncthreads();
@@ -892,12 +894,11 @@ cudaError_t launchRenderMode(const RenderArgs& a, cudaStream_t s) {
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         // as many resident threads per SM for either tile size
         const uint32_t grid = uint32_t(sms) * kPersistentBlocksPerSm * (kRenderThreads / threads);
-        renderPersistentKernel<MODE, CAP, TILE, STATS, GATHER>
-            <<<grid < a.totalTiles ? grid : a.totalTiles, threads, smem, s>>>(a, map);
-    } else {
-        renderKernel<MODE, CAP, TILE, STATS, GATHER><<<a.tileLaunch ? a.tileLaunch : a.totalTiles, threads, smem, s>>>(a, map);
+        return launchDependent(renderPersistentKernel<MODE, CAP, TILE, STATS, GATHER>,
+                               dim3(grid < a.totalTiles ? grid : a.totalTiles), threads, smem, s, a, map);
     }
-    return cudaGetLastError();
+    return launchDependent(renderKernel<MODE, CAP, TILE, STATS, GATHER>, dim3(a.tileLaunch ? a.tileLaunch : a.totalTiles),
+                           threads, smem, s, a, map);
 }
 
 // the window capacity for K: 4, 16 or 64 register slots

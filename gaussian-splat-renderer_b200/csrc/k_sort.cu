@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(256) sortHistKernel(const __grid_constant__ So
     __shared__ uint32_t sHist[kMaxSortPasses][D::kBins];
     __shared__ uint32_t sLast;
     __shared__ uint32_t sActive[kMaxSortPasses];
+    gridWait();
     DeviceControl* ctl = a.ctl;
     const uint32_t entries = a.frameMode == 2 ? a.count : ctl->c.entries;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(256) sortHistKernel(const __grid_constant__ So
 #pragma unroll
             for (int j = 0; j < kHistItems; ++j) {
                 const uint32_t idx = base + j * 256 + threadIdx.x;
-                k[j] = idx < runEnd ? __ldg(&keys[idx]) : 0ull;
+                k[j] = idx < runEnd ? __ldcg(&keys[idx]) : 0ull;
             }
 #pragma unroll
             for (int j = 0; j < kHistItems; ++j) {
@@ -202,7 +203,7 @@ __global__ void __launch_bounds__(256) sortHistKernel(const __grid_constant__ So
 #pragma unroll
             for (int j = 0; j < kHistItems; ++j) {
                 const uint32_t idx = base + j * 256 + threadIdx.x;
-                k[j] = idx < entries ? __ldg(&keys[idx]) : 0ull;
+                k[j] = idx < entries ? __ldcg(&keys[idx]) : 0ull;
             }
 #pragma unroll
             for (int j = 0; j < kHistItems; ++j) {
@@ -429,8 +430,8 @@ __device__ __forceinline__ void sortPassTiles(const SortArgs& a, uint32_t p, uns
 #pragma unroll
     for (int j = 0; j < kItems; ++j) {
         const uint32_t idx = itemBase + j * 32;
-        key[j] = idx < tileEnd ? __ldg(&keysIn[idx]) : ~0ull;
-        if (PAIRS) val[PAIRS ? j : 0] = idx < tileEnd ? __ldg(&valsIn[idx]) : 0u;
+        key[j] = idx < tileEnd ? __ldcg(&keysIn[idx]) : ~0ull;
+        if (PAIRS) val[PAIRS ? j : 0] = idx < tileEnd ? __ldcg(&valsIn[idx]) : 0u;
     }
     uint32_t* wc = sWarpCnt + warp * kBins;
 #pragma unroll
@@ -536,6 +537,7 @@ __global__ void __launch_bounds__(kSortThreads, BITS == 9 ? 2 : 3) sortPassKerne
                                                                                  uint32_t p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t sOff[1 << BITS], sScan[8], sTile;
+    gridWait();
     const SortPlan* plan = a.plan;
     if (!plan->active[p]) return;
     if (plan->packed) sortPassTiles<false, 24, BITS>(a, p, smem, sOff, sScan, sTile);
@@ -550,6 +552,7 @@ __global__ void __launch_bounds__(kSortThreads, BITS == 9 ? 2 : 4) depthPassKern
                                                                                   uint32_t p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t sOff[1 << BITS], sScan[8], sTile;
+    gridWait();
     if (!a.plan->active[p]) return;
     sortPassTiles<false, kDepthSortItems, BITS, true>(a, p, smem, sOff, sScan, sTile);
 }
@@ -560,6 +563,7 @@ __global__ void __launch_bounds__(kSortThreads, BITS == 9 ? 2 : 4) depthPassKern
 // the next one starts (or at the list's end).
 constexpr uint32_t kRangeItems = 8;
 __global__ void __launch_bounds__(256) rangesKernel(const __grid_constant__ RenderArgs a) {
+    gridWait();
     const DeviceControl* ctl = a.ctl;
     const uint32_t n = ctl->c.entries;
     const uint64_t* keys = a.keys[ctl->c.sorted_buffer & 1u];
@@ -573,7 +577,7 @@ __global__ void __launch_bounds__(256) rangesKernel(const __grid_constant__ Rend
             const uint4* v = reinterpret_cast<const uint4*>(keys + base);
 #pragma unroll
             for (uint32_t j = 0; j < kRangeItems / 2; ++j) {
-                const uint4 w = __ldg(&v[j]);
+                const uint4 w = __ldcg(&v[j]);
                 t[2 * j] = uint32_t(((uint64_t(w.y) << 32) | w.x) >> shift);
                 t[2 * j + 1] = uint32_t(((uint64_t(w.w) << 32) | w.z) >> shift);
             }
@@ -607,12 +611,13 @@ __global__ void __launch_bounds__(256) rangesKernel(const __grid_constant__ Rend
 // ---- standalone exclusive scan (GpuScan plain / kNonZero / kGather) ---------------------------
 constexpr int kScanItems = int(kScanBlockItems / 256);
 static_assert(256 * kScanItems == int(kScanBlockItems), "one scan block = 256 threads x kScanItems");
-__global__ void __launch_bounds__(256) scanKernel(const uint32_t* __restrict__ in, const uint32_t* __restrict__ index,
-                                                  uint32_t* __restrict__ out, uint32_t* total, uint32_t count,
+__global__ void __launch_bounds__(256) scanKernel(const uint32_t* in, const uint32_t* index, uint32_t* __restrict__ out,
+                                                  uint32_t* total, uint32_t count,
                                                   uint32_t mode, uint64_t* status, DeviceControl* ctl,
                                                   uint32_t setupCapacity, uint32_t waitSite,
                                                   const __grid_constant__ ScanGather gather) {
     __shared__ uint32_t sBlock, sWarp[8], sExclusive;
+    gridWait();
     const uint64_t* words = mode == kScanGatherSorted ? gather.words[gather.plan->sortedBuffer & 1u] : nullptr;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) sBlock = atomicAdd(&ctl->tickets[12], 1u);
@@ -712,14 +717,17 @@ cudaError_t launchSortBits(const SortArgs& a, uint32_t histBlocks, cudaStream_t 
     }
     const bool depth = a.frameMode == 2;
     const uint32_t tiles = a.maxTiles < 1 ? 1 : a.maxTiles;  // of kSortTile = kDepthSortTile = a histogram chunk
-    sortHistKernel<BITS><<<histBlocks < 1 ? 1 : (histBlocks < tiles ? histBlocks : tiles), 256, 0, s>>>(a);
+    cudaError_t e = launchDependent(sortHistKernel<BITS>, dim3(histBlocks < 1 ? 1 : (histBlocks < tiles ? histBlocks : tiles)),
+                                    256, 0, s, a);
+    if (e != cudaSuccess) return e;
     const uint32_t limit = uint32_t(depth ? depthGrid : passGrid);
     const uint32_t grid = tiles < limit ? tiles : limit;
     for (uint32_t p = 0; p < a.passesLaunched; ++p) {
-        if (depth) depthPassKernel<BITS><<<grid, kSortThreads, kDepthSmem, s>>>(a, p);
-        else sortPassKernel<BITS><<<grid, kSortThreads, kListSmem, s>>>(a, p);
+        e = depth ? launchDependent(depthPassKernel<BITS>, dim3(grid), kSortThreads, kDepthSmem, s, a, p)
+                  : launchDependent(sortPassKernel<BITS>, dim3(grid), kSortThreads, kListSmem, s, a, p);
+        if (e != cudaSuccess) return e;
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 }  // namespace
@@ -736,8 +744,7 @@ cudaError_t launchSort(const SortArgs& a, uint32_t histBlocks, cudaStream_t s) {
 }
 
 cudaError_t launchRanges(const RenderArgs& a, uint32_t capacity, cudaStream_t s) {
-    rangesKernel<<<gridFor((capacity + kRangeItems - 1) / kRangeItems, 256, 148 * 16), 256, 0, s>>>(a);
-    return cudaGetLastError();
+    return launchDependent(rangesKernel, dim3(gridFor((capacity + kRangeItems - 1) / kRangeItems, 256, 148 * 16)), 256, 0, s, a);
 }
 
 cudaError_t launchScan(const uint32_t* in, const uint32_t* index, uint32_t* out, uint32_t* total, uint32_t count,
@@ -749,6 +756,9 @@ cudaError_t launchScan(const uint32_t* in, const uint32_t* index, uint32_t* out,
         return cudaSuccess;
     }
     const ScanGather g = gather ? *gather : ScanGather{{nullptr, nullptr}, nullptr, 0};
+    if (setupCapacity)  // a frame's scan, behind the frame's kernel before it
+        return launchDependent(scanKernel, dim3(blocks), 256, 0, s, in, index, out, total, count, mode, status, ctl,
+                               setupCapacity, waitSite, g);
     scanKernel<<<blocks, 256, 0, s>>>(in, index, out, total, count, mode, status, ctl, setupCapacity, waitSite, g);
     return cudaGetLastError();
 }

@@ -6,6 +6,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <utility>
 
 #include "gsr_types.h"
 
@@ -19,6 +20,26 @@ inline std::atomic<T>& perDevice(std::atomic<T> (&table)[64]) {
     int dev = 0;
     cudaGetDevice(&dev);
     return table[dev & 63];
+}
+
+// Launches a kernel that starts with gridWait() behind the stream's last kernel: its launch is
+// processed while that one runs and its blocks wait for the completion instead of the whole launch
+// (programmatic dependent launch). Frames launched kernel by kernel: 10,000 gaussians 116 -> 97 us,
+// 1.24 M at 1080p 551 -> 520 us, 6 M at 4K 2.18 -> 2.15 ms. Captured frames measure the same.
+template <class... Params, class... Args>
+inline cudaError_t launchDependent(void (*kernel)(Params...), dim3 grid, uint32_t threads, size_t smem, cudaStream_t s,
+                                   Args&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
 struct DevCameraArgs {  // = DevCamera (splat_math.cuh)
