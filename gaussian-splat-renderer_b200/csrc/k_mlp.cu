@@ -14,10 +14,15 @@
 //               over the chunk's samples (activations transposed by ldmatrix.trans), kept in
 //               registers across the chunks and written once as the block's partial sums (no
 //               atomics: the run is reproducible bit for bit)
-//   adamStep    one thread per parameter: the batch gradient from the partial sums, Adam
+//               A step is a serial chain (14 small products a chunk, four chunks, then Adam), 36 us at
+//               batch 65,536 (88 before the weight image, the sample copies a chunk ahead, the bias
+//               columns' hoisted addresses and Adam's spread loads; same bits)
+//   adamStep    one thread per parameter: the batch gradient from the partial sums, Adam, the weight
+//               image's next state
 //   encode      latents of every gaussian (fp32 encoder, stored fp16)
 //   gate        per gaussian, the tensor-core decode on its directions against the SH colour;
 //               max channel error above the gate -> fallback (the latent's last half = NaN)
+#include "gsr_device.cuh"
 #include "kernels.cuh"
 #include "mlp.cuh"
 #include "splat_math.cuh"
@@ -33,17 +38,67 @@ constexpr int kTcWarps = 4, kTcThreads = kTcWarps * 32, kTcChunk = kTcWarps * 16
 constexpr int kTcBlockSamples = kTcChunk * kTcChunks;
 constexpr int S48 = kEncIn + 8, S64 = kEncHidden + 8, S32 = kMlpHidden + 8, S16 = 16 + 8;
 
-struct alignas(16) TrainSmem {
+// The weights as a block holds them in shared memory: BF16 in both operand layouts (padding zero) and
+// the fp32 biases. One image in device memory, made once a training call and kept current by the
+// Adam kernel parameter by parameter, so that a block's copy is 16-byte transfers (each block used
+// to convert and transpose the fp32 masters, 7 us of a step).
+struct alignas(16) TrainWeights {
     // forward operands [n][k] (the weight matrices transposed), backward operands [n][k] = W[in][out]
     __nv_bfloat16 wt1e[kEncHidden][S48], wt2e[8][S64], wt1d[kMlpHidden][S16], wt2d[kMlpHidden][S32], wt3d[8][S32];
     __nv_bfloat16 wb3[kMlpHidden][S16], wb2[kMlpHidden][S32], wb1[kMlpLatent][S32], wb2e[kEncHidden][S16];
+    float b1e[kEncHidden], b2e[8], b1d[kMlpHidden], b2d[kMlpHidden], b3d[8];
+};
+static_assert(sizeof(TrainWeights) % 16 == 0 && sizeof(TrainWeights) <= kColorTrainImageBytes, "the weight image");
+
+// Parameter p's places in the image.
+__device__ __forceinline__ void storeWeight(TrainWeights& W, int p, float v) {
+    using L = MlpLayout;
+    const __nv_bfloat16 b = __float2bfloat16_rn(v);
+    if (p < L::kEncB1) {
+        W.wt1e[p % kEncHidden][p / kEncHidden] = b;
+    } else if (p < L::kEncW2) {
+        W.b1e[p - L::kEncB1] = v;
+    } else if (p < L::kEncB2) {
+        const int i = (p - L::kEncW2) / kMlpLatent, o = (p - L::kEncW2) % kMlpLatent;
+        W.wt2e[o][i] = b;
+        W.wb2e[i][o] = b;
+    } else if (p < L::kDecW1) {
+        W.b2e[p - L::kEncB2] = v;
+    } else if (p < L::kDecB1) {
+        const int i = (p - L::kDecW1) / kMlpHidden, o = (p - L::kDecW1) % kMlpHidden;
+        W.wt1d[o][i] = b;
+        if (i < kMlpLatent) W.wb1[i][o] = b;  // the latent rows of W1d
+    } else if (p < L::kDecW2) {
+        W.b1d[p - L::kDecB1] = v;
+    } else if (p < L::kDecB2) {
+        const int i = (p - L::kDecW2) / kMlpHidden, o = (p - L::kDecW2) % kMlpHidden;
+        W.wt2d[o][i] = b;
+        W.wb2[i][o] = b;
+    } else if (p < L::kDecW3) {
+        W.b2d[p - L::kDecB2] = v;
+    } else if (p < L::kDecB3) {
+        const int i = (p - L::kDecW3) / kMlpOut, o = (p - L::kDecW3) % kMlpOut;
+        W.wt3d[o][i] = b;
+        W.wb3[i][o] = b;
+    } else {
+        W.b3d[p - L::kDecB3] = v;
+    }
+}
+
+constexpr int kSampleStride = kEncIn + 4;  // floats: 16-byte reads of neighbouring rows fall into distinct banks
+struct alignas(16) TrainSmem : TrainWeights {
     // the chunk's activations and gradients, one row per sample
     __nv_bfloat16 x[kTcChunk][S48], h[kTcChunk][S64], in[kTcChunk][S16], a1[kTcChunk][S32], a2[kTcChunk][S32];
     __nv_bfloat16 dO[kTcChunk][S16], dA2[kTcChunk][S32], dA1[kTcChunk][S32], dZ[kTcChunk][S16], dH[kTcChunk][S64];
-    float b1e[kEncHidden], b2e[8], b1d[kMlpHidden], b2d[kMlpHidden], b3d[8];
+    float sample[kTcChunk][kSampleStride];  // the next chunk's SH coefficients
     float tgt[kTcChunk][4];
     float lossWarp[kTcWarps];
 };
+
+__global__ void packTrainKernel(const float* __restrict__ params, TrainWeights* out) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < MlpLayout::kCount) storeWeight(*out, p, params[p]);
+}
 
 __device__ __forceinline__ uint32_t mix32(uint32_t x) {
     x ^= x >> 16;
@@ -76,9 +131,9 @@ struct TrainArgs {
     uint32_t count;
     uint32_t dirs;           // directions per gaussian
     uint32_t seed;
-    const float* params;     // fp32 masters [kCount]
+    const TrainWeights* weights;
     float* partials;         // [blocks][kCount + 1] (the last float: the block's loss sum)
-    const uint32_t* step;    // current step (device counter, advanced by adamStep)
+    uint32_t step;           // the step's number, which keys its samples
 };
 
 __device__ __forceinline__ uint32_t smemAddr(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
@@ -164,54 +219,40 @@ __global__ void __launch_bounds__(kTcThreads) trainStepKernel(const __grid_const
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(smemRaw);
     using L = MlpLayout;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3;
-    const float* P = a.params;
     auto bf = [](float v) { return __float2bfloat16_rn(v); };
-    // weights in both layouts (padding zero), biases, and the constant zero columns
-    for (int e = tid; e < kEncHidden * S48; e += kTcThreads) {
-        const int o = e / S48, i = e % S48;
-        S.wt1e[o][i] = bf(i < kEncIn ? P[L::kEncW1 + i * kEncHidden + o] : 0.0f);
-    }
-    for (int e = tid; e < 8 * S64; e += kTcThreads) {
-        const int o = e / S64, i = e % S64;
-        S.wt2e[o][i] = bf(i < kEncHidden ? P[L::kEncW2 + i * kMlpLatent + o] : 0.0f);
-    }
-    for (int e = tid; e < kMlpHidden * S16; e += kTcThreads) {
-        const int o = e / S16, i = e % S16;
-        S.wt1d[o][i] = bf(i < kMlpIn ? P[L::kDecW1 + i * kMlpHidden + o] : 0.0f);
-        S.wb3[o][i] = bf(i < kMlpOut ? P[L::kDecW3 + o * kMlpOut + i] : 0.0f);
-    }
-    for (int e = tid; e < kMlpHidden * S32; e += kTcThreads) {
-        const int r = e / S32, c = e % S32;
-        S.wt2d[r][c] = bf(c < kMlpHidden ? P[L::kDecW2 + c * kMlpHidden + r] : 0.0f);
-        S.wb2[r][c] = bf(c < kMlpHidden ? P[L::kDecW2 + r * kMlpHidden + c] : 0.0f);
-    }
-    for (int e = tid; e < 8 * S32; e += kTcThreads) {
-        const int r = e / S32, c = e % S32;
-        S.wt3d[r][c] = bf(r < kMlpOut && c < kMlpHidden ? P[L::kDecW3 + c * kMlpOut + r] : 0.0f);
-        S.wb1[r][c] = bf(c < kMlpHidden ? P[L::kDecW1 + r * kMlpHidden + c] : 0.0f);  // the latent rows of W1d
-    }
-    for (int e = tid; e < kEncHidden * S16; e += kTcThreads) {
-        const int r = e / S16, c = e % S16;
-        S.wb2e[r][c] = bf(c < kMlpLatent ? P[L::kEncW2 + r * kMlpLatent + c] : 0.0f);
-    }
-    for (int e = tid; e < kEncHidden; e += kTcThreads) S.b1e[e] = P[L::kEncB1 + e];
-    for (int e = tid; e < kMlpHidden; e += kTcThreads) {
-        S.b1d[e] = P[L::kDecB1 + e];
-        S.b2d[e] = P[L::kDecB2 + e];
-    }
-    if (tid < 8) {
-        S.b2e[tid] = P[L::kEncB2 + tid];
-        S.b3d[tid] = tid < kMlpOut ? P[L::kDecB3 + tid] : 0.0f;
-    }
+    // Sample tid of a chunk (tid < 64): its gaussian's coefficients on their way to shared memory, its
+    // degree and direction. A chunk ahead of their use (the first one ahead of the wait for the
+    // weights): fetched at the chunk's start they were 4 us of its 15.
+    const uint32_t step = a.step;
+    int degree = 0;
+    uint32_t gaussian = 0, dirIndex = 0;
+    auto fetch = [&](int chunk) {
+        if (tid >= kTcChunk) return;
+        const uint32_t k = blockIdx.x * kTcBlockSamples + chunk * kTcChunk + tid;
+        gaussian = uint32_t((uint64_t(hash3(a.seed, step, k)) * a.count) >> 32);
+        dirIndex = hash3(a.seed ^ 0x5bd1e995u, step, k) % a.dirs;
+        const float4* src = reinterpret_cast<const float4*>(a.sh + size_t(gaussian) * kEncIn);
+#pragma unroll
+        for (int q = 0; q < kEncIn / 4; ++q)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smemAddr(&S.sample[tid][4 * q])), "l"(src + q)
+                         : "memory");
+        degree = int(a.degrees[gaussian]);
+    };
+    fetch(0);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    gridWait();
+    for (int e = tid; e < int(sizeof(TrainWeights) / 16); e += kTcThreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smemAddr(reinterpret_cast<uint4*>(static_cast<TrainWeights*>(&S)) + e)),
+                     "l"(reinterpret_cast<const uint4*>(a.weights) + e) : "memory");
     for (int e = tid; e < kTcChunk * 8; e += kTcThreads) {
         const int r = e / 8, c = 8 + e % 8;
         S.in[r][c] = bf(0.0f);  // columns 11..15 stay zero (8..10 are rewritten per chunk)
         S.dO[r][c] = bf(0.0f);
         S.dZ[r][c] = bf(0.0f);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 
-    const uint32_t step = *a.step;
     const int rb = warp * 16;
     float acc[kTilesPerWarp][4];
 #pragma unroll
@@ -219,28 +260,27 @@ __global__ void __launch_bounds__(kTcThreads) trainStepKernel(const __grid_const
     float bsum[2] = {0.0f, 0.0f};  // bias gradients of columns tid and tid + 128 of [dH | dZ | dA1 | dA2 | dO]
     float loss = 0.0f;
     for (int chunk = 0; chunk < kTcChunks; ++chunk) {
-        // ---- the chunk's samples: (gaussian, direction), SH coefficients and the SH colour
+        // ---- the chunk's samples: their direction and SH colour (threads 0..63), their coefficients
+        // as the encoder's input (threads 64..127)
         if (tid < kTcChunk) {
-            const uint32_t k = blockIdx.x * kTcBlockSamples + chunk * kTcChunk + tid;
-            const uint32_t gs = uint32_t((uint64_t(hash3(a.seed, step, k)) * a.count) >> 32);
-            const uint32_t jd = hash3(a.seed ^ 0x5bd1e995u, step, k) % a.dirs;
             float dir[3], target[3];
-            sampleDirection(gs, jd, dir);
-            const float* shg = a.sh + size_t(gs) * kEncIn;
-            evalSH(int(a.degrees[gs]), shg, dir[0], dir[1], dir[2], target);
-            const float4* sh4 = reinterpret_cast<const float4*>(shg);
-#pragma unroll
-            for (int q = 0; q < kEncIn / 4; ++q) {
-                const float4 v = __ldg(&sh4[q]);
-                *reinterpret_cast<uint32_t*>(&S.x[tid][4 * q]) = packBf16(v.x, v.y);
-                *reinterpret_cast<uint32_t*>(&S.x[tid][4 * q + 2]) = packBf16(v.z, v.w);
-            }
+            sampleDirection(gaussian, dirIndex, dir);
+            evalSH(degree, S.sample[tid], dir[0], dir[1], dir[2], target);
             for (int c = 0; c < 3; ++c) {
                 S.in[tid][kMlpLatent + c] = bf(dir[c]);
                 S.tgt[tid][c] = target[c];
             }
+        } else {
+            const int row = tid - kTcChunk;
+#pragma unroll
+            for (int q = 0; q < kEncIn / 4; ++q) {
+                const float4 v = *reinterpret_cast<const float4*>(&S.sample[row][4 * q]);
+                *reinterpret_cast<uint32_t*>(&S.x[row][4 * q]) = packBf16(v.x, v.y);
+                *reinterpret_cast<uint32_t*>(&S.x[row][4 * q + 2]) = packBf16(v.z, v.w);
+            }
         }
         __syncthreads();
+        if (chunk + 1 < kTcChunks) fetch(chunk + 1);
         // ---- forward, each warp its 16 rows
         {
             float c[8][4];
@@ -351,21 +391,24 @@ __global__ void __launch_bounds__(kTcThreads) trainStepKernel(const __grid_const
                 default: gradTimes(acc[q], S.a2, gt.m0, S.dO, gt.n0); break;
             }
         }
+        // (the column's rows added in order; its place is looked up once, not at every row, which was
+        // 7 us of a chunk)
 #pragma unroll
         for (int h2 = 0; h2 < 2; ++h2) {
             const int col = tid + h2 * kTcThreads;
+            if (col >= 139) break;
+            const __nv_bfloat16* at = col < 64    ? &S.dH[0][col]
+                                      : col < 72  ? &S.dZ[0][col - 64]
+                                      : col < 104 ? &S.dA1[0][col - 72]
+                                      : col < 136 ? &S.dA2[0][col - 104]
+                                                  : &S.dO[0][col - 136];
+            const int stride = col < 64 ? S64 : col < 72 ? S16 : col < 136 ? S32 : S16;
             float sum = 0.0f;
-            for (int r = 0; r < kTcChunk; ++r) {
-                const __nv_bfloat16 v = col < 64    ? S.dH[r][col]
-                                        : col < 72  ? S.dZ[r][col - 64]
-                                        : col < 104 ? S.dA1[r][col - 72]
-                                        : col < 136 ? S.dA2[r][col - 104]
-                                        : col < 139 ? S.dO[r][col - 136]
-                                                    : __float2bfloat16_rn(0.0f);
-                sum += __bfloat162float(v);
-            }
+#pragma unroll 16
+            for (int r = 0; r < kTcChunk; ++r) sum += __bfloat162float(at[r * stride]);
             bsum[h2] += sum;
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");  // the next chunk's samples
         __syncthreads();  // the next chunk overwrites the rows
     }
     // ---- the block's partial sums
@@ -412,30 +455,49 @@ struct AdamArgs {
     uint32_t blocks;   // partial sums per parameter
     float invBatch;
     float lr, beta1, beta2, eps;
+    TrainWeights* weights;  // the step's result as the next step reads it
     uint32_t* step;    // advanced here (t = step + 1 in the bias corrections)
     float* lossOut;    // mean squared error per pair of steps lossBase .. maxSteps - 1
     uint32_t lossBase;
     uint32_t maxSteps;
 };
 
-__global__ void adamStepKernel(const __grid_constant__ AdamArgs a) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp a block, 163 of them, so that the loads of the partial sums (added in order, one after
+// another) come from every SM, 64 of a thread in flight: 16 -> 10 us for 256 blocks' sums (caches cold).
+constexpr int kAdamThreads = 32;
+__global__ void __launch_bounds__(kAdamThreads) adamStepKernel(const __grid_constant__ AdamArgs a) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    gridWait();
+    const uint32_t p = blockIdx.x * kAdamThreads + threadIdx.x;
     const uint32_t step = *a.step;
     if (p <= uint32_t(MlpLayout::kCount)) {
         float g = 0.0f;
-        for (uint32_t b = 0; b < a.blocks; ++b) g += a.partials[size_t(b) * (MlpLayout::kCount + 1) + p];
+        const float* part = a.partials + p;
+        constexpr uint32_t kStride = MlpLayout::kCount + 1, kDeep = 64;
+        uint32_t b = 0;
+        for (; b + kDeep <= a.blocks; b += kDeep) {
+            float v[kDeep];
+#pragma unroll
+            for (uint32_t k = 0; k < kDeep; ++k) v[k] = __ldcg(part + size_t(b + k) * kStride);
+#pragma unroll
+            for (uint32_t k = 0; k < kDeep; ++k) g += v[k];
+        }
+        for (; b < a.blocks; ++b) g += __ldcg(part + size_t(b) * kStride);
         g *= a.invBatch;
         if (p == uint32_t(MlpLayout::kCount)) {
             if (step >= a.lossBase && step < a.maxSteps) a.lossOut[step - a.lossBase] = g / 3.0f;  // per channel
         } else {
             const float t = float(step + 1);
-            const float m = a.beta1 * a.m[p] + (1.0f - a.beta1) * g;
-            const float v = a.beta2 * a.v[p] + (1.0f - a.beta2) * g * g;
+            // (the roundings spelled out: which product is fused decides the last bit)
+            const float m = __fmaf_rn(a.beta1, a.m[p], __fmul_rn(1.0f - a.beta1, g));
+            const float v = __fmaf_rn(a.beta2, a.v[p], __fmul_rn(__fmul_rn(1.0f - a.beta2, g), g));
             a.m[p] = m;
             a.v[p] = v;
             const float mh = m / (1.0f - powf(a.beta1, t));
             const float vh = v / (1.0f - powf(a.beta2, t));
-            a.params[p] -= a.lr * mh / (sqrtf(vh) + a.eps);
+            const float w = a.params[p] - a.lr * mh / (sqrtf(vh) + a.eps);
+            a.params[p] = w;
+            storeWeight(*a.weights, int(p), w);
         }
     }
     __syncthreads();
@@ -571,9 +633,17 @@ __global__ void __launch_bounds__(kGateWarps * 32) gateKernel(const __grid_const
 
 }  // namespace
 
+cudaError_t launchPackTrain(const float* params, void* image, cudaStream_t s) {
+    const cudaError_t e = cudaMemsetAsync(image, 0, sizeof(TrainWeights), s);  // the operands' padding
+    if (e != cudaSuccess) return e;
+    packTrainKernel<<<(MlpLayout::kCount + 127) / 128, 128, 0, s>>>(params, static_cast<TrainWeights*>(image));
+    return cudaGetLastError();
+}
+
 cudaError_t launchColorTrainStep(const float* sh, const uint8_t* degrees, uint32_t count, uint32_t dirs, uint32_t seed,
-                                 uint32_t batch, float* params, float* m, float* v, float* partials, uint32_t* step,
-                                 float lr, float* lossOut, uint32_t lossBase, uint32_t maxSteps, cudaStream_t s) {
+                                 uint32_t batch, float* params, float* m, float* v, float* partials, void* image,
+                                 uint32_t stepIndex, uint32_t* step, float lr, float* lossOut, uint32_t lossBase,
+                                 uint32_t maxSteps, cudaStream_t s) {
     static std::atomic<bool> configuredOn[64] = {};
     std::atomic<bool>& configured = perDevice(configuredOn);
     const int smem = int(sizeof(TrainSmem));
@@ -583,12 +653,14 @@ cudaError_t launchColorTrainStep(const float* sh, const uint8_t* degrees, uint32
         configured = true;
     }
     const uint32_t blocks = batch / kTcBlockSamples;
-    TrainArgs ta{sh, degrees, count, dirs, seed, params, partials, step};
-    trainStepKernel<<<blocks, kTcThreads, smem, s>>>(ta);
-    AdamArgs aa{params, m, v, partials, blocks, 1.0f / float(batch), lr, 0.9f, 0.999f, 1e-8f, step, lossOut, lossBase,
-                maxSteps};
-    adamStepKernel<<<(MlpLayout::kCount + 1 + 255) / 256, 256, 0, s>>>(aa);
-    return cudaGetLastError();
+    TrainWeights* weights = static_cast<TrainWeights*>(image);
+    TrainArgs ta{sh, degrees, count, dirs, seed, weights, partials, stepIndex};
+    const cudaError_t e = launchDependent(trainStepKernel, dim3(blocks), kTcThreads, smem, s, ta);
+    if (e != cudaSuccess) return e;
+    AdamArgs aa{params, m, v, partials, blocks, 1.0f / float(batch), lr, 0.9f, 0.999f, 1e-8f, weights, step, lossOut,
+                lossBase, maxSteps};
+    return launchDependent(adamStepKernel, dim3((MlpLayout::kCount + 1 + kAdamThreads - 1) / kAdamThreads), kAdamThreads,
+                           0, s, aa);
 }
 
 cudaError_t launchColorEncode(const float* sh, const float* params, uint4* latents, DecoderWeights* decoder,

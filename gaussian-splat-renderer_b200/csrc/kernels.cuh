@@ -68,6 +68,7 @@ static_assert(sizeof(DevView) == 32, "DevView layout");
 struct DecoderWeights;
 constexpr size_t kDecoderWeightsBytes = 32 * 16 * 2 + 32 * 32 * 2 + 8 * 32 * 2 + (32 + 32 + 8) * 4;
 constexpr uint32_t kColorModelParams = 5195;
+constexpr size_t kColorTrainImageBytes = 24 * 1024;
 
 struct SceneArgs {
     const uint4* b0;     // soa posAlpha | geometry records | aos records
@@ -244,11 +245,15 @@ cudaError_t launchScan(const uint32_t* in, const uint32_t* index, uint32_t* out,
 // Decoded SH coefficients [count][48] (zeros past each gaussian's evaluated degree) and degrees.
 cudaError_t launchShDecode(const SceneArgs& scene, uint32_t geometry, uint32_t color, uint32_t count, int evalDegree,
                            float* out, uint8_t* degrees, cudaStream_t s);
+// The training step's weight image (kColorTrainImageBytes) from the fp32 parameters.
+cudaError_t launchPackTrain(const float* params, void* image, cudaStream_t s);
 // One training step (batch pairs, a multiple of colorTrainBatchMultiple()): forward/backward
-// partial sums, then Adam; step = {step counter, scratch counter} advanced on the device.
+// partial sums, then Adam, which also renews the weight image; step = {step counter, scratch
+// counter} advanced on the device, stepIndex its value before this step.
 cudaError_t launchColorTrainStep(const float* sh, const uint8_t* degrees, uint32_t count, uint32_t dirs, uint32_t seed,
-                                 uint32_t batch, float* params, float* m, float* v, float* partials, uint32_t* step,
-                                 float lr, float* lossOut, uint32_t lossBase, uint32_t maxSteps, cudaStream_t s);
+                                 uint32_t batch, float* params, float* m, float* v, float* partials, void* image,
+                                 uint32_t stepIndex, uint32_t* step, float lr, float* lossOut, uint32_t lossBase,
+                                 uint32_t maxSteps, cudaStream_t s);
 // The tensor-core decoder packed from the fp32 parameters.
 cudaError_t launchPackDecoder(const float* params, struct DecoderWeights* decoder, cudaStream_t s);
 uint32_t colorTrainBatchMultiple();

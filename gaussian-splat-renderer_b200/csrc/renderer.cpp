@@ -1810,7 +1810,8 @@ namespace {
 int trainColorModel(const GsrSceneDesc& scene, GsrColorModel& m, uint32_t steps) {
     const GsrColorModelOptions& o = m.options;
     const uint32_t n = scene.count, blocks = o.batch / colorTrainBatchMultiple();
-    DevBuf sh, degrees, partials, lossDev, counters;
+    DevBuf sh, degrees, partials, image, lossDev, counters;
+    GSR_CUDA(image.alloc(kColorTrainImageBytes));
     GSR_CUDA(sh.alloc(size_t(n) * 48 * 4));
     GSR_CUDA(degrees.alloc(n));
     GSR_CUDA(partials.alloc(size_t(blocks) * (kColorModelParams + 1) * 4));
@@ -1830,10 +1831,11 @@ int trainColorModel(const GsrSceneDesc& scene, GsrColorModel& m, uint32_t steps)
     if (ce == cudaSuccess) ce = cudaEventRecord(e0, s);
     if (ce == cudaSuccess)
         ce = launchShDecode(sceneArgs(scene), scene.geometry, scene.color, n, m.degree, sh.as<float>(), degrees.as<uint8_t>(), s);
+    if (ce == cudaSuccess) ce = launchPackTrain(m.params.as<float>(), image.p, s);
     for (uint32_t k = 0; ce == cudaSuccess && k < steps; ++k)
         ce = launchColorTrainStep(sh.as<float>(), degrees.as<uint8_t>(), n, o.directions, o.seed, o.batch,
                                   m.params.as<float>(), m.mom.as<float>(), m.vel.as<float>(), partials.as<float>(),
-                                  m.stepDev.as<uint32_t>(), o.learning_rate, lossDev.as<float>(), m.step, m.step + steps, s);
+                                  image.p, m.step + k, m.stepDev.as<uint32_t>(), o.learning_rate, lossDev.as<float>(), m.step, m.step + steps, s);
     if (ce == cudaSuccess)
         ce = launchColorEncode(sh.as<float>(), m.params.as<float>(), m.latents.as<uint4>(), m.decoder.as<DecoderWeights>(), n, s);
     if (ce == cudaSuccess)
