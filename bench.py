@@ -295,6 +295,9 @@ def pass_bytes(scene_format: str, ctl, n: int, tiles: int, bits: int = 8, views:
       offsets and span hints again and 8 bytes per list entry (emission).
     tile sort: histogram read + a read and a write of every entry per active pass.
     ranges: every entry read, 8 bytes per tile written.
+    A list built row by row (its runs counted in the control block's first extension word) has
+      other bytes: scan + emission are the sorted words, the hints of the visible and 8 bytes a
+      run; the tile sort reads the runs twice and writes 4 bytes an entry and every tile's range.
     A frame of several views (n = views x the scene's gaussians records) reads the scene once:
     every gaussian's position, shape and SH (the union of the views' reads), then the writes of
     every record."""
@@ -308,6 +311,15 @@ def pass_bytes(scene_format: str, ctl, n: int, tiles: int, bits: int = 8, views:
         pre = sum(per_g) * (n // views)
     pre += 4 * n + 8 * n + 64 * vis
     per_entry = 16 if ctl.packed_entries else 24
+    runs = getattr(ctl, "ext_pad", [0])[0]
+    if runs:
+        return {
+            "preprocess": float(pre),
+            "depth sort": float(8 * n + 16 * n * depth_sort_passes(ctl, bits)),
+            "scan + emission": float(8 * n + 16 * vis + 8 * runs),
+            "tile sort": float(2 * 8 * runs + 4 * m + 8 * tiles),
+            "ranges": 0.0,
+        }
     return {
         "preprocess": float(pre),
         "depth sort": float(8 * n + 16 * n * depth_sort_passes(ctl, bits)),

@@ -26,18 +26,21 @@ enum WaitSite : uint32_t {
 };
 
 constexpr int kControlTickets = 32;
-constexpr uint32_t kListSortTickets = 1, kDepthSortTickets = 16;
+constexpr uint32_t kListSortTickets = 1, kDepthSortTickets = 16, kRowCutTicket = 14, kRowPartTicket = 15;
 
 // The per-frame control block in device memory (GsrControl in gsr_b200.h) plus scratch
 // counters that only the kernels use.
 struct DeviceControl {
     GsrControl c;
     // block tickets: [1 + p] list sort pass p, [12] scans, [13] the rasterizer's tile queue,
-    // [16 + p] depth sort pass p (binning mode)
+    // [16 + p] depth sort pass p (binning mode), [14] the row plan's cut, [15] the row partition
     uint32_t tickets[kControlTickets];
     uint32_t histDone[2];       // blocks of the histogram kernels that have finished (list, depth sort)
+    uint32_t rowCutSlot;        // row-wise list: the depth-sorted record the full list ends in (all ones: none)
+    uint32_t rowCutTiles;       // ... and the tiles of it that are kept
     uint32_t forceTimeout;      // test hook: look-back waits see no predecessor for this many spins
-    uint32_t pad[5];
+    uint32_t spillCursor;       // row-wise list: the spilled runs taken so far
+    uint32_t pad[2];
 };
 
 // Items of one block of the exclusive scan (scanKernel: 256 threads x kScanItems); the scan's

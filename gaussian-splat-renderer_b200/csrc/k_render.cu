@@ -474,9 +474,9 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a,
     range.y = range.y < entries ? range.y : entries;
     range.x = range.x < range.y ? range.x : range.y;
     const uint32_t sortedBuffer = a.ctl->c.sorted_buffer & 1u;
-    const uint32_t* values = a.values[sortedBuffer];
+    const uint32_t* values = a.list ? a.list : a.values[sortedBuffer];
     const uint64_t* packedKeys = a.keys[sortedBuffer];
-    const bool packed = a.plan->packed != 0;
+    const bool packed = !a.list && a.plan->packed != 0;
     const uint64_t indexMask = (1ull << a.plan->indexBits) - 1ull;
     const float4* records = reinterpret_cast<const float4*>(a.splats) + size_t(view) * a.count * 3;
     const uint4* records32 = reinterpret_cast<const uint4*>(a.packed) + size_t(view) * a.count * 2;

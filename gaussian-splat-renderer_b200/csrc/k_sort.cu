@@ -296,48 +296,6 @@ __global__ void __launch_bounds__(256) sortHistKernel(const __grid_constant__ So
 }
 
 // ---- one onesweep pass ------------------------------------------------------------------------
-// Decoupled look-back of digit d for tile t: the sum of the digit's counts over tiles 0..t-1
-// (status words [tile][BINS]). Eight predecessors are read per round trip; a word that is not
-// yet published (or carries an older frame's epoch) stops the window and is re-read after a
-// short sleep. Waits are bounded by kSpinLimit (then the timeout is reported and the partial
-// sum returned).
-template <int BINS>
-__device__ __forceinline__ uint32_t digitLookback(const uint64_t* status, uint32_t t, uint32_t d, uint32_t epoch,
-                                                  DeviceControl* ctl) {
-    constexpr int kWindow = 8;
-    const uint32_t forced = ctl->forceTimeout;
-    uint32_t exclusive = 0, spins = 0;
-    int q = int(t) - 1;
-    while (q >= 0) {
-        uint64_t w[kWindow];
-#pragma unroll
-        for (int j = 0; j < kWindow; ++j)
-            w[j] = q - j >= 0 ? ldRelaxed(&status[size_t(q - j) * BINS + d]) : packStatus(epoch, kFlagInclusive, 0);
-        int used = 0;
-        bool found = false;
-#pragma unroll
-        for (int j = 0; j < kWindow; ++j) {
-            if (found || used != j) continue;
-            bool ready = statusReady(w[j], epoch);
-            if (forced && spins < forced) ready = false;  // test hook: behave as if nobody published
-            if (!ready) continue;
-            exclusive += uint32_t(w[j]);
-            ++used;
-            if (statusFlag(w[j]) == kFlagInclusive) found = true;
-        }
-        if (found) break;
-        q -= used;
-        if (used < kWindow) {
-            if (++spins >= kSpinLimit || (forced && spins >= forced)) {
-                reportTimeout(ctl, kWaitSort);
-                break;
-            }
-            __nanosleep(32);
-        }
-    }
-    return exclusive;
-}
-
 // One pass over 256-thread tiles of kItems keys per thread. PAIRS = false: the entries are
 // single words (vkey << indexBits | index), 24 per thread; PAIRS = true: (tile << 32 | depth)
 // keys with a 32-bit value array, 16 per thread. The frame launches both and the one that does

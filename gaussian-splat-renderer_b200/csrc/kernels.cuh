@@ -117,6 +117,20 @@ struct FrontArgs {
     uint32_t recordBits;                  // bits of a record index (V * N - 1)
     uint32_t depthViewShift;              // the view's field in the depth words, above the depth bits
                                           // (0: none; the depth sort then orders all views together)
+    // binning by tile rows (rowRecords != 0): the tile rows' entry counts and their buckets, see k_rows.cu
+    uint32_t rowRecords;                  // 1: the frame's list is built row by row
+    uint32_t rowsPerView;                 // the tile rows of the tallest view
+    const uint32_t* buckets;              // [bucketCount] view << 8 | row: the frame's tile rows
+    uint32_t bucketCount;
+    unsigned long long* rowHist;          // [viewCount][kRowBins] row entries << 32 | tiles, of every record
+    unsigned long long* rowKept;          // the same of the records kept by an overflowing list
+    uint4* rowPlan;                       // [viewCount][kRowBins] a bucket's first row entry and count, first tile entry and count
+    uint32_t* rowStatus;                  // [viewCount * ceil(N / kRowPartTile)][kRowBins] look-back words of the partition
+    uint2* rowEntries;                    // [capacity] (x0 | x1 << 16, gaussian), bucket by bucket
+    uint32_t* spill;                      // [spillCapacity] runs of records with more than kSpanRows rows
+    uint32_t spillCapacity;
+    uint32_t* list;                       // [capacity] the list: gaussians, tile by tile
+    uint32_t* ranges;                     // uint2 per frame tile
     const uint4* latents;                 // learned colour: fp16 latents [N] (null: SH colour)
     const struct DecoderWeights* decoder; // learned colour: the tensor-core decoder (mlp.cuh)
     float4* decoded;                      // tcgen05 decode: kept gaussians' colours [viewCount][N]
@@ -124,6 +138,14 @@ struct FrontArgs {
     DeviceControl* ctl;
     LogfFixups logf;
 };
+
+// Tile rows of a view at most; the depth-sorted records of one block of the cut; the fewest of one block
+// of the partition (its look-back words are sized by them).
+constexpr uint32_t kRowBins = 256;
+constexpr uint32_t kRowTile = 1024;
+constexpr uint32_t kRowPartTile = 512;
+constexpr uint32_t kSpillPerBlock = 512;  // spilled runs of a preprocess block (256 records) of its own
+constexpr uint32_t kRowMaxTilesX = 512;  // tiles of a row at most (a block's counters)
 
 // Sort plan written by the histogram kernel's last block.
 constexpr int kMaxSortPasses = 10;  // 64 key bits in 7-bit digits
@@ -190,6 +212,7 @@ struct RenderArgs {
     uint32_t bounds;          // GsrTileBounds of the list (32 x 8 tiles clip splats to their 16-px rectangle)
     const uint32_t* values[2];
     const uint64_t* keys[2];
+    const uint32_t* list;     // the list built row by row (null: keys / values of the sort)
     uint32_t* ranges;         // uint2 per tile of the frame (all views)
     void* image;              // per view W*H at the view's pixelBase: float4, half4 or uchar4 (imageFormat)
     uint32_t imageFormat;     // 0: float4, 1: half4 (fp16 round to nearest even), 2: uchar4 (lround(clamp(v) 255))
@@ -216,12 +239,19 @@ constexpr uint32_t kTileStatListLength = 0, kTileStatFetched = 1, kTileStatEvalu
 // ---- launchers (return cudaGetLastError()) ---------------------------------------------------
 cudaError_t launchFrameBegin(DeviceControl* ctl, uint32_t count, uint32_t capacity, uint32_t* ranges,
                              uint32_t rangeWords, SortPlan* plan, uint32_t forceTimeout, cudaStream_t s,
-                             SortPlan* plan2 = nullptr, uint32_t* clearWords = nullptr, uint32_t clearCount = 0);
+                             SortPlan* plan2 = nullptr, uint32_t* clearWords = nullptr, uint32_t clearCount = 0,
+                             uint4* clearVec4s = nullptr, uint32_t clearVec4Count = 0);
+// A row-wise frame's partition: the records of a block.
+uint32_t rowPartitionTile(uint64_t records);
 cudaError_t launchFront(const FrontArgs& a, uint32_t geometry, uint32_t color, cudaStream_t s);
 // Binning mode, split around the depth sort: preprocess + the depth keys, then (after the sort of
 // the depth keys) the scan of the counts in depth order and the emission in that order.
 cudaError_t launchFrontBinningKeys(const FrontArgs& a, uint32_t geometry, uint32_t color, cudaStream_t s);
 cudaError_t launchFrontBinningEmit(const FrontArgs& a, cudaStream_t s);
+// The same list built row by row (k_rows.cu), in the place of launchFrontBinningEmit, the tile sort and
+// the ranges: the records in depth order into the tile rows' buckets, then each bucket by tile.
+cudaError_t launchRowPartition(const FrontArgs& a, cudaStream_t s);
+cudaError_t launchRowTiles(const FrontArgs& a, uint32_t maxTilesX, cudaStream_t s);
 // The learned colour's decode as a pre-pass on the tcgen05 tensor cores: every kept gaussian's
 // colour for every view of the frame into a.decoded (before the preprocess, which reads them).
 cudaError_t launchDecodeColoursTc(const FrontArgs& a, uint32_t geometry, cudaStream_t s);

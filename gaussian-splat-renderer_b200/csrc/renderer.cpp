@@ -449,8 +449,34 @@ struct GsrRenderer {
     DevBuf control, plan;
     // binning mode: the records' depth words (ping-pong), their sort's look-back words and plan
     DevBuf depthKeys[2], depthStatus, depthPlan;
-    // the depth sort's per-view digit counts and bases, [views][depthPasses()][1 << digitBits] each
+    // the depth sort's per-view digit counts and bases, [views][depthPasses()][1 << digitBits] each,
+    // behind the tile rows' sizes of a row-wise list (rowHistWords: of every record, of the kept ones)
     DevBuf depthRuns;
+    DevBuf buckets;  // view << 8 | row of every tile row of the frame
+    // A row-wise list's work for allocViews views: the look-back words of the partition, the buckets, the
+    // runs of splats of many rows (each preprocess block's own, and a common million).
+    DevBuf rowWork;
+    size_t rowStatusBytes(size_t v) const { return v * ((size_t(scene.count) + kRowPartTile - 1) / kRowPartTile) * kRowBins * 4; }
+    size_t spillRuns(size_t v) const { return v * ((size_t(scene.count) + 255) / 256) * kSpillPerBlock + (1u << 20); }
+    bool rowWise = false;       // the current layout's list is built row by row (k_rows.cu)
+    uint32_t maxTilesX = 0, maxTilesY = 0;
+    // The row-wise list wants at most kRowBins rows a view and kRowMaxTilesX tiles a row (a block's
+    // counters), and enough rows for the records: a row is built by eight blocks, so few rows of many
+    // records leave the chip idle. Frames, row by row against sorted (us): 133,000 records a row
+    // (4 M at 640 x 480) 743 against 782, 155,000 (1.24 M at 1280 x 128) 466 against 495, 250,000
+    // (4 M at 256 x 256) 684 against 654.
+    bool rowWiseFits(uint32_t v) const {
+        return binning() && maxTilesY <= kRowBins && maxTilesX <= kRowMaxTilesX &&
+               uint64_t(scene.count) * v <= kRowMaxRecords * totalRows;
+    }
+    uint64_t totalRows = 0;
+    static constexpr uint64_t kRowMaxRecords = 196608;
+    uint32_t rowHistWords() const { return allocViews * kRowBins * 2 * 2; }
+    uint32_t rowStatusVec4s(uint32_t v) const {
+        const uint64_t tile = rowPartitionTile(uint64_t(scene.count) * v);
+        return uint32_t(v * ((scene.count + tile - 1) / tile) * (kRowBins / 4));
+    }
+    uint32_t rowTiles(size_t v) const { return uint32_t(v * ((size_t(scene.count) + kRowTile - 1) / kRowTile)); }
     bool binning() const { return settings.list_mode == GSR_LIST_BINNING; }
     // the radix digit width of both sorts, and the depth sort's passes: its keys are the varying
     // depth bits and the no-tile bit, at most 32 bits (depths are positive floats)
@@ -645,6 +671,16 @@ struct GsrRenderer {
         return c - c % kBlockSize;
     }
 
+    // What only a sorted list needs: the look-back words of its passes and the records' offsets.
+    int sortedListReady(List& l) {
+        if (!l.status.p) {
+            GSR_CUDA(l.status.alloc(size_t(l.passes) * l.maxTiles * statusWordsPerTile() * 8));
+            GSR_CUDA(cudaMemset(l.status.p, 0, l.status.bytes));
+        }
+        if (!offsets.p) GSR_CUDA(offsets.alloc(size_t(scene.count) * allocViews * 4));
+        return GSR_OK;
+    }
+
     int createList(uint32_t capacity, std::unique_ptr<List>& out) {
         auto l = std::make_unique<List>();
         l->capacity = capacity;
@@ -654,8 +690,10 @@ struct GsrRenderer {
             GSR_CUDA(l->keys[b].alloc(size_t(capacity) * 8));
             if (!binning()) GSR_CUDA(l->values[b].alloc(size_t(capacity) * 4));  // binning entries are one word
         }
-        GSR_CUDA(l->status.alloc(size_t(l->passes) * l->maxTiles * statusWordsPerTile() * 8));
-        GSR_CUDA(cudaMemset(l->status.p, 0, l->status.bytes));
+        if (!rowWise) {
+            const int rc = sortedListReady(*l);
+            if (rc) return rc;
+        }
         GSR_CUDA(cudaEventCreateWithFlags(&l->lastUse, cudaEventDisableTiming));
         out = std::move(l);
         return GSR_OK;
@@ -685,12 +723,13 @@ struct GsrRenderer {
             for (auto& k : depthKeys) GSR_CUDA(k.alloc(n * 8));
             GSR_CUDA(depthStatus.alloc(size_t(depthPasses()) * depthTiles(v) * statusWordsPerTile() * 8));
             GSR_CUDA(cudaMemset(depthStatus.p, 0, depthStatus.bytes));
-            GSR_CUDA(depthRuns.alloc(size_t(depthRunWords(v)) * 2 * 4));
+            GSR_CUDA(depthRuns.alloc(size_t(v) * kRowBins * 2 * 2 * 4 + size_t(depthRunWords(v)) * 2 * 4));
             GSR_CUDA(cudaMemset(depthRuns.p, 0, depthRuns.bytes));
+            GSR_CUDA(rowWork.alloc(rowStatusBytes(v) + size_t(v) * kRowBins * 16 + spillRuns(v) * 4));
         }
         GSR_CUDA(tileCounts.alloc(n * 4));
-        GSR_CUDA(offsets.alloc(n * 4));
-        GSR_CUDA(scanStatus.alloc((n + 255) / 256 * 8));
+        offsets.release();  // (sortedListReady)
+        GSR_CUDA(scanStatus.alloc(std::max<size_t>((n + 255) / 256, rowTiles(v)) * 8));
         GSR_CUDA(cudaMemset(scanStatus.p, 0, scanStatus.bytes));
         for (auto& s : slots) {
             if (s->camHost) cudaFreeHost(s->camHost);
@@ -728,6 +767,8 @@ struct GsrRenderer {
         std::vector<DevView> dv(v);
         uint32_t tileBase = 0;
         uint64_t pixelBase = 0;
+        maxTilesX = maxTilesY = 0;
+        totalRows = 0;
         for (uint32_t i = 0; i < v; ++i) {
             GsrViewLayout& L = views[i];
             L.width = w[i];
@@ -736,18 +777,29 @@ struct GsrRenderer {
             L.tiles_y = (h[i] + tileH() - 1) / tileH();
             L.tile_base = tileBase;
             L.pixel_base = pixelBase;
+            maxTilesX = std::max(maxTilesX, L.tiles_x);
+            maxTilesY = std::max(maxTilesY, L.tiles_y);
+            totalRows += L.tiles_y;
             dv[i] = DevView{L.tile_base, L.tiles_x, L.tiles_y, L.width, L.height, 0, L.pixel_base};
             tileBase += L.tiles_x * L.tiles_y;
             pixelBase += uint64_t(w[i]) * h[i];
         }
         totalTiles = uint32_t(tiles);
         totalPixels = pixels;
+        rowWise = rowWiseFits(v);
         width = views[0].width;
         height = views[0].height;
         tilesX = views[0].tiles_x;
         tilesY = views[0].tiles_y;
         GSR_CUDA(viewsDevice.alloc(sizeof(DevView) * v));
         GSR_CUDA(cudaMemcpy(viewsDevice.p, dv.data(), sizeof(DevView) * v, cudaMemcpyHostToDevice));
+        if (rowWise) {
+            std::vector<uint32_t> b;
+            for (uint32_t i = 0; i < v; ++i)
+                for (uint32_t row = 0; row < views[i].tiles_y; ++row) b.push_back((i << 8) | row);
+            GSR_CUDA(buckets.alloc(b.size() * 4));
+            GSR_CUDA(cudaMemcpy(buckets.p, b.data(), b.size() * 4, cudaMemcpyHostToDevice));
+        }
         const uint32_t tileCount = totalTiles;
         GSR_CUDA(ranges.alloc(size_t(tileCount) * 8));
         GSR_CUDA(cudaMemset(ranges.p, 0, ranges.bytes));
@@ -775,6 +827,7 @@ struct GsrRenderer {
             rc = createList(initial, list);
             if (rc) return rc;
         }
+        if (!rowWise) return sortedListReady(*list);
         return GSR_OK;
     }
 
@@ -911,8 +964,8 @@ struct GsrRenderer {
         slot.frameIndex = frameIndex;
         // frameBegin, preprocess, scan, duplicate, histogram, one per pass, ranges, render
         // binning: frameBegin, preprocess, depth histogram + passes, scan, duplicate, list
-        // histogram + passes, ranges, render
-        kernelLaunches += (binning() ? 8 + depthPasses() + list->passes : 7 + list->passes) + (split ? uint32_t(parts.size()) - 1 : 0) +
+        // histogram + passes, ranges, render; row by row: ... the row plan, partition and tiles, render
+        kernelLaunches += (rowWise ? 7 + depthPasses() : binning() ? 8 + depthPasses() + list->passes : 7 + list->passes) + (split ? uint32_t(parts.size()) - 1 : 0) +
                           (colorLatents && tcDecode() ? 1u : 0u);
         timed = timing;
         ++frameIndex;
@@ -931,10 +984,13 @@ struct GsrRenderer {
         mark(stream);
         GSR_CUDA(cudaMemcpyAsync(slot.camDevice.p, slot.camHost, sizeof(DevCameraArgs) * viewCount,
                                  cudaMemcpyHostToDevice, stream));
-        GSR_CUDA(launchFrameBegin(ctl, scene.count * viewCount, l.capacity, ranges.as<uint32_t>(), tileCount * 2,
-                                  sortPlan, forceTimeout, stream, binning() ? depthPlan.as<SortPlan>() : nullptr,
+        // (a row-wise list writes every tile's range)
+        GSR_CUDA(launchFrameBegin(ctl, scene.count * viewCount, l.capacity, ranges.as<uint32_t>(),
+                                  rowWise ? 0u : tileCount * 2, sortPlan, forceTimeout, stream,
+                                  binning() ? depthPlan.as<SortPlan>() : nullptr,
                                   binning() ? depthRuns.as<uint32_t>() : nullptr,
-                                  binning() ? depthRunWords(viewCount) : 0u));
+                                  binning() ? rowHistWords() + depthRunWords(viewCount) : 0u,
+                                  rowWise ? rowWork.as<uint4>() : nullptr, rowWise ? rowStatusVec4s(viewCount) : 0u));
         FrontArgs fa{};
         fa.cam = slot.camDevice.as<DevCameraArgs>();
         fa.views = viewsDevice.as<DevView>();
@@ -973,6 +1029,21 @@ struct GsrRenderer {
             fa.recordBits = recordBits();
             const uint32_t viewBits = depthViewBits(viewCount);
             fa.depthViewShift = viewBits ? fa.recordBits + 32u : 0u;
+            if (rowWise) {
+                fa.rowRecords = 1;
+                fa.rowsPerView = maxTilesY;
+                fa.buckets = buckets.as<uint32_t>();
+                fa.bucketCount = uint32_t(totalRows);
+                fa.rowHist = depthRuns.as<unsigned long long>();
+                fa.rowKept = fa.rowHist + size_t(allocViews) * kRowBins;
+                fa.rowStatus = rowWork.as<uint32_t>();
+                fa.rowPlan = reinterpret_cast<uint4*>(rowWork.as<unsigned char>() + rowStatusBytes(allocViews));
+                fa.spill = reinterpret_cast<uint32_t*>(fa.rowPlan + size_t(allocViews) * kRowBins);
+                fa.spillCapacity = uint32_t(spillRuns(allocViews));
+                fa.rowEntries = l.keys[0].as<uint2>();
+                fa.list = l.keys[1].as<uint32_t>();
+                fa.ranges = ranges.as<uint32_t>();
+            }
             GSR_CUDA(launchFrontBinningKeys(fa, scene.geometry, scene.color, stream));
             mark(stream);
             // each view's records by (depth, record index): 32 depth bits above the record index,
@@ -991,11 +1062,11 @@ struct GsrRenderer {
             sd.indexBits = fa.recordBits;
             sd.segments = viewCount;
             sd.segLength = scene.count;
-            sd.segHist = depthRuns.as<uint32_t>();
-            sd.segBase = depthRuns.as<uint32_t>() + depthRunWords(allocViews);
+            sd.segHist = depthRuns.as<uint32_t>() + rowHistWords();
+            sd.segBase = sd.segHist + depthRunWords(allocViews);
             GSR_CUDA(launchSort(sd, 148 * 2, stream));
             mark(stream);
-            GSR_CUDA(launchFrontBinningEmit(fa, stream));
+            GSR_CUDA(rowWise ? launchRowPartition(fa, stream) : launchFrontBinningEmit(fa, stream));
         } else {
             GSR_CUDA(launchFront(fa, scene.geometry, scene.color, stream));
         }
@@ -1016,7 +1087,8 @@ struct GsrRenderer {
         sa.binning = binning() ? 1u : 0u;
         sa.tileCount = tileCount;
         sa.count = scene.count;
-        GSR_CUDA(launchSort(sa, 148 * 4, stream));
+        if (rowWise) GSR_CUDA(launchRowTiles(fa, maxTilesX, stream));
+        else GSR_CUDA(launchSort(sa, 148 * 4, stream));
         mark(stream);
 
         RenderArgs ra{};
@@ -1049,7 +1121,8 @@ struct GsrRenderer {
             ra.testedPairs = testedPairs.as<unsigned long long>();
             GSR_CUDA(cudaMemsetAsync(testedPairs.p, 0, 8, stream));
         }
-        GSR_CUDA(launchRanges(ra, l.capacity, stream));
+        if (rowWise) ra.list = l.keys[1].as<uint32_t>();
+        else GSR_CUDA(launchRanges(ra, l.capacity, stream));
         mark(stream);
         // the images may still be on their way to the host (the streaming call): wait for it
         if (int rc = waitCopied(imageCopied, stream)) return rc;
@@ -1524,7 +1597,31 @@ int gsr_read_list(GsrRenderer* r, uint32_t* keysLo, uint32_t* keysHi, uint32_t* 
     const uint32_t b = c.sorted_buffer & 1u;
     SortPlan plan;
     GSR_CUDA(cudaMemcpy(&plan, r->plan.p, sizeof(plan), cudaMemcpyDeviceToHost));
-    if (n && (keysLo || keysHi || (values && plan.packed))) {
+    if (n && r->rowWise) {
+        // the list holds the gaussians, the ranges the tiles, the records the depths
+        std::vector<uint32_t> g(n), rng(size_t(r->totalTiles) * 2), depth;
+        GSR_CUDA(cudaMemcpy(g.data(), r->list->keys[1].p, size_t(n) * 4, cudaMemcpyDeviceToHost));
+        GSR_CUDA(cudaMemcpy(rng.data(), r->ranges.p, rng.size() * 4, cudaMemcpyDeviceToHost));
+        if (keysLo) {
+            const size_t records = size_t(r->scene.count) * r->views.size();
+            depth.resize(records);
+            if (r->settings.render_splat == GSR_RENDER_SPLAT_FULL)
+                GSR_CUDA(cudaMemcpy2D(depth.data(), 4, static_cast<const unsigned char*>(r->splats.p) + 8, 48, 4, records,
+                                      cudaMemcpyDeviceToHost));
+            else
+                GSR_CUDA(cudaMemcpy(depth.data(), r->depths.p, records * 4, cudaMemcpyDeviceToHost));
+        }
+        size_t view = 0;
+        for (uint32_t t = 0; t < r->totalTiles; ++t) {
+            while (view + 1 < r->views.size() && r->views[view + 1].tile_base <= t) ++view;
+            for (uint32_t i = rng[2 * size_t(t)]; i < std::min(rng[2 * size_t(t) + 1], n); ++i) {
+                const size_t at = view * r->scene.count + g[i];
+                if (keysHi) keysHi[i] = t;
+                if (keysLo) keysLo[i] = g[i] < r->scene.count ? depth[at] : 0u;
+                if (values) values[i] = g[i];
+            }
+        }
+    } else if (n && (keysLo || keysHi || (values && plan.packed))) {
         std::vector<uint64_t> k(n);
         GSR_CUDA(cudaMemcpy(k.data(), r->list->keys[b].p, size_t(n) * 8, cudaMemcpyDeviceToHost));
         // packed words: (((tile << W) | depth mod 2^W) << indexBits) | index; the depth bits above
@@ -1565,7 +1662,7 @@ int gsr_read_list(GsrRenderer* r, uint32_t* keysLo, uint32_t* keysHi, uint32_t* 
             if (keysHi) keysHi[i] = hi;
         }
     }
-    if (n && values && !plan.packed)
+    if (n && values && !r->rowWise && !plan.packed)
         GSR_CUDA(cudaMemcpy(values, r->list->values[b].p, size_t(n) * 4, cudaMemcpyDeviceToHost));
     if (rangesOut) {
         const uint32_t words = std::min<uint32_t>(rangesWords, r->totalTiles * 2);

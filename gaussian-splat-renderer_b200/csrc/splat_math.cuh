@@ -397,32 +397,36 @@ __device__ __forceinline__ uint32_t coverageCount(const Coverage& cv, const RowG
 // x0 | x1 << 16, the second array's four words rows 3-6.
 constexpr int kSpanRows = 7;
 constexpr uint32_t kSpanMarker = 0x7FC00000u;
+// row-wise lists: the runs of a record with more rows are in the frame's spilled runs; the hint's words
+// y and z hold the row count and the first run's index
+constexpr uint32_t kSpanSpilled = 0x00080000u;
 __device__ __forceinline__ bool isSpanHint(const float4& h) {
     return (__float_as_uint(h.x) & 0xFFC00000u) == kSpanMarker;
 }
 
-// coverageCount that also stores the rows' runs of a span hint (spanForm: rows <= kSpanRows and
-// the grid's width below 65536) into `hint` (rows 0-2, words 1-3) and `more` (rows 3-6).
-__device__ __forceinline__ uint32_t coverageCountSpans(const Coverage& cv, const RowGeom& g, const BinShape& S, int gx,
-                                                       uint32_t* hint, uint32_t* more, int& r0, int& rows,
-                                                       bool& spanForm) {
-    int r1;
-    coverageRows(cv, S, r0, r1);
-    rows = r1 - r0;
-    spanForm = r1 - r0 <= kSpanRows && gx < 65536 && r0 >= 0 && r0 < 65536;
-    uint32_t n = 0;
-    for (int r = r0; r < r1; ++r) {
-        int x0, x1;
-        coverageRowSpan(cv, g, r, S, x0, x1);
-        n += uint32_t(x1 - x0);
-        if (spanForm) {
-            const int k = r - r0;
-            const uint32_t w = uint32_t(x0) | (uint32_t(x1) << 16);
-            if (k < 3) hint[1 + k] = w;
-            else more[k - 3] = w;
-        }
-    }
-    return n;
+// What a row's run is computed from (coverageRowSpan's inputs), as a warp's lanes pass it around.
+struct RowTerms {
+    float cx, cy, A, B, D, eyPad, eyRight0, At, pad;
+    uint32_t binsX;      // x0 | x1 << 16
+    uint32_t useEllipse;
+};
+constexpr uint32_t kRowTermWords = 11;
+__device__ __forceinline__ RowTerms rowTerms(const Coverage& cv, const RowGeom& g) {
+    return RowTerms{cv.e.cx, cv.e.cy, cv.e.A, cv.e.B, cv.e.D, cv.e.eyPad, g.eyRight0, g.At, g.pad,
+                    uint32_t(cv.bins.x0) | (uint32_t(imax(cv.bins.x0, cv.bins.x1)) << 16), cv.useEllipse ? 1u : 0u};
+}
+__device__ __forceinline__ void rowTermsSpan(const RowTerms& t, int row, const BinShape& S, int& x0, int& x1) {
+    Coverage cv;
+    cv.bins = BinRect{int(t.binsX & 0xFFFFu), 0, int(t.binsX >> 16), 0};
+    cv.useEllipse = t.useEllipse != 0;
+    cv.e.cx = t.cx;
+    cv.e.cy = t.cy;
+    cv.e.A = t.A;
+    cv.e.B = t.B;
+    cv.e.D = t.D;
+    cv.e.eyPad = t.eyPad;
+    const RowGeom g{0.0f, t.eyRight0, t.At, t.pad};
+    coverageRowSpan(cv, g, row, S, x0, x1);
 }
 
 // What the key emission needs of a visible gaussian's coverage beyond its record, kept by the

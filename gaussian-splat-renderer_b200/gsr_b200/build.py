@@ -32,8 +32,8 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off", f"-I{INCLUDE}", f"-I{CSRC}"]
 # translation units whose floating-point results must match the reference bit for bit
 # (the rasterizer's image is held to a tolerance instead and uses FMA and the hardware exp2)
-EXACT_UNITS = {"k_front.cu", "k_encode.cu"}
-CU_UNITS = ["k_front.cu", "k_sort.cu", "k_render.cu", "k_encode.cu", "k_mlp.cu"]
+EXACT_UNITS = {"k_front.cu", "k_rows.cu", "k_encode.cu"}
+CU_UNITS = ["k_front.cu", "k_rows.cu", "k_sort.cu", "k_render.cu", "k_encode.cu", "k_mlp.cu"]
 HOST_UNITS = ["renderer.cpp", "ply_loader.cpp", "training_cameras.cpp", "scene_io_abi.cpp", "color_checkpoint.cpp"]
 
 

@@ -280,7 +280,7 @@ typedef struct GsrControl {
     uint32_t status;                 /* GsrControlStatus bits */
     uint32_t timeout_where;          /* id of the wait that gave up */
     uint32_t epoch;                  /* frame counter of the device-side look-back flags */
-    uint32_t sort_passes;            /* radix passes that moved data */
+    uint32_t sort_passes;            /* radix passes that moved data (a list built row by row: 1) */
     uint32_t key_bits;               /* significant bits of the (tile | depth) key */
     uint32_t depth_low_bits;         /* depth bits that vary across the frame's keys */
     uint32_t depth_min_bits, depth_max_bits;
@@ -289,7 +289,7 @@ typedef struct GsrControl {
     uint32_t capacity;               /* list capacity of this frame */
     uint32_t packed_entries;         /* 1: entries were single 64-bit words (tile|depth|index) */
     uint32_t index_bits;             /* bits of the gaussian index in a packed entry */
-    uint32_t ext_pad[3];
+    uint32_t ext_pad[3];             /* [0]: the (splat, tile row) runs of a list built row by row, else 0 */
 } GsrControl;
 
 /* ---- the renderer (SplatTileRenderer) ---------------------------------------------------- */
