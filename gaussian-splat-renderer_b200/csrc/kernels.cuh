@@ -256,6 +256,10 @@ cudaError_t launchRowTiles(const FrontArgs& a, uint32_t maxTilesX, cudaStream_t 
 // colour for every view of the frame into a.decoded (before the preprocess, which reads them).
 cudaError_t launchDecodeColoursTc(const FrontArgs& a, uint32_t geometry, cudaStream_t s);
 cudaError_t launchSort(const SortArgs& a, uint32_t histBlocks, cudaStream_t s);
+// The depth sort (frameMode 2) of runs short enough for a cluster's shared memory, in one launch and in
+// place (plan->sortedBuffer = 0): whether the frame's runs are, and the launch.
+bool depthSortInCluster(uint32_t records, uint32_t runs);
+cudaError_t launchDepthSortCluster(const SortArgs& a, cudaStream_t s);
 cudaError_t launchRanges(const RenderArgs& a, uint32_t capacity, cudaStream_t s);
 cudaError_t launchRender(const RenderArgs& a, cudaStream_t s);
 cudaError_t launchLogfTable(float* out, LogfFixups t, cudaStream_t s);

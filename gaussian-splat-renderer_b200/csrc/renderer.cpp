@@ -1079,7 +1079,10 @@ struct GsrRenderer {
         // frameBegin, preprocess, scan, duplicate, histogram, one per pass, ranges, render
         // binning: frameBegin, preprocess, depth histogram + passes, scan, duplicate, list
         // histogram + passes, ranges, render; row by row: ... the row plan, partition and tiles, render
-        kernelLaunches += (rowWise ? 7 + depthPasses() : binning() ? 8 + depthPasses() + list->passes : 7 + list->passes) + (split ? uint32_t(parts.size()) - 1 : 0) +
+        // (the depth sort of short runs is one launch)
+        const uint32_t depthLaunches = depthSortInCluster(scene.count, uint32_t(views.size())) ? 1u : 1u + depthPasses();
+        kernelLaunches += (rowWise ? 6 + depthLaunches : binning() ? 7 + depthLaunches + list->passes : 7 + list->passes) +
+                          (split ? uint32_t(parts.size()) - 1 : 0) +
                           (colorLatents && tcDecode() ? 1u : 0u);
         timed = timing;
         ++frameIndex;
@@ -1178,7 +1181,8 @@ struct GsrRenderer {
             sd.segLength = scene.count;
             sd.segHist = depthRuns.as<uint32_t>() + rowHistWords();
             sd.segBase = sd.segHist + depthRunWords(allocViews);
-            GSR_CUDA(launchSort(sd, 148 * 2, stream));
+            GSR_CUDA(depthSortInCluster(scene.count, viewCount) ? launchDepthSortCluster(sd, stream)
+                                                                : launchSort(sd, 148 * 2, stream));
             mark(stream);
             GSR_CUDA(rowWise ? launchRowPartition(fa, stream) : launchFrontBinningEmit(fa, stream));
         } else {
