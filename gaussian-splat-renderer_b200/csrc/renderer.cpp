@@ -1,13 +1,14 @@
 // Host side of the B200 splat-tiles path: the C ABI of include/gsr_b200.h over a C++ renderer
 // that mirrors gsr::SplatTileRenderer (src/render/splat_tile_renderer.h:143-290) and
 // gsr::GpuScene (src/render/gpu_scene.h:42-78), launching the kernels of k_front.cu,
-// k_sort.cu, k_render.cu and k_encode.cu on the caller's stream.
+// k_sort.cu, k_rows.cu, k_render.cu and k_encode.cu on the caller's stream.
 //
 // Per frame (render):
 //   frameBegin   reset of the control block + tile ranges      (splat_tile_renderer.cpp:653-661)
 //   front        preprocess + count + scan + setup + duplicate (passes 1, 2, 6, 7)
 //   sort         histogram/plan + onesweep passes               (pass 8, global 64-bit keys)
 //   ranges       per-tile [start, end)                          (pass 9)
+//   or, in binning mode, preprocess, depth sort, and the list and its ranges row by row (k_rows.cu)
 //   render       the tile rasterizer                            (pass 10)
 //   readback     control block -> the frame slot's pinned buffer, read frames_in_flight later
 //
@@ -386,6 +387,11 @@ cudaError_t uploadHost(const std::vector<Upload>& parts) {
         if (e != cudaSuccess) failed.store(int(e));
     };
     try {
+        pieces.reserve(total / Stager::kPiece + parts.size());
+    } catch (...) {
+        return uploadPlain(parts);
+    }
+    try {
         for (const Upload& u : parts)
             for (size_t o = 0; o < u.bytes; o += Stager::kPiece)
                 pieces.push_back(Upload{static_cast<unsigned char*>(u.dst) + o, static_cast<const unsigned char*>(u.src) + o,
@@ -393,9 +399,8 @@ cudaError_t uploadHost(const std::vector<Upload>& parts) {
         const unsigned n = std::max(1u, std::min(Stager::kThreads, std::thread::hardware_concurrency()));
         threads.reserve(n);
         for (unsigned t = 1; t < n; ++t) threads.emplace_back(work, t);
-    } catch (...) {  // no memory or no thread: those that run do the work, with this one
+    } catch (...) {  // (of the threads: those that run do the work, with this one)
     }
-    if (pieces.empty()) return uploadPlain(parts);
     work(0);
     for (std::thread& t : threads) t.join();
     return cudaError_t(failed.load());
