@@ -3,6 +3,8 @@
 //   frameBegin   reset of the control block and the tile ranges
 //   preprocess   per gaussian: scene decode, near/opacity culls, cov3D, EWA cov2D, conic/radius,
 //                pixel centre, 16-px rectangle, SH colour, tight tile count (streaming, no waits)
+//                and, in binning mode, the tiles of every tile row (k_rows.cu builds the list from there;
+//                the two kernels below serve the global mode and the layouts its rule excludes)
 //   scan         exclusive prefix of the counts in index order (GpuScan, k_sort.cu) = the list
 //                offsets, whose last block clamps the list to the capacity (tile_setup)
 //   duplicate    per gaussian: one (tile << 32 | depth bits, index) entry per covered tile
@@ -511,8 +513,9 @@ __global__ void __launch_bounds__(kFrontThreads, 4) preprocessKernel(const __gri
     }
     // The runs of the warp's splats, one (splat, row) pair a lane at a time: a splat has about two rows and
     // the longest of 32 has eight or more, so a lane walking its own rows left most lanes idle (preprocess
-    // of 1.24 M gaussians 141 -> 125 us, of eight views 890 -> 788, of 6 M at 4K 531 -> 460). The terms go through shared memory, under the splat's
-    // place among those with rows; the SH staging area is free once the warp's colours are done.
+    // of 1.24 M gaussians 141 -> 125 us, of eight views 890 -> 788, of 6 M at 4K 531 -> 460). The terms go
+    // through shared memory, under the splat's place among those with rows; the SH staging area is free once
+    // the warp's colours are done.
     if (a.bounds != kBoundsRect && __any_sync(0xFFFFFFFFu, rows != 0)) {
         if (staged && !shStageReady()) waitShStage(a.ctl, false);  // (a forced expiry reads on before the copy has landed)
         uint32_t* terms = reinterpret_cast<uint32_t*>(gShStage) + (tid >> 5) * (staged ? 32u * 48u : 32u * kRunWords);

@@ -14,6 +14,8 @@
 // and ~235 for match.any.sync over random 8-bit digits (measured on B200 with a synthetic
 // throughput loop).
 //
+// A frame's short depth sorts take one launch instead (depthClusterKernel).
+//
 // Key shortening: the list key is (tile << 32 | depth bits). All depth bits above the highest
 // bit where the frame's smallest and largest depth differ are equal for every key, and so are
 // the tile bits above the largest tile id; the sort therefore orders the "virtual key"

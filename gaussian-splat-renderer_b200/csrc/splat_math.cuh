@@ -7,7 +7,7 @@
 //   src/splat/splat_math.cpp  quaternionToMatrix, computeCov3D, computeCov2D, projectToPixel,
 //                             conicAndRadius, computeTileRect, evalSH, preprocessGaussian
 //   src/splat/tile_coverage.cpp  makeCutoffEllipse, ellipseRows, ellipseRowBounds,
-//                             ellipseRowSpan, rectToBins, makeCoverage, coverageCount
+//                             ellipseRowSpan, rectToBins, makeCoverage
 //   shaders/splat_preprocess.comp:147-223  the GPU culls (NaN-safe near test, o < 1/255)
 #pragma once
 
@@ -373,20 +373,6 @@ __device__ __forceinline__ void coverageRowSpan(const Coverage& cv, const RowGeo
     const int c = imin(cv.bins.x1, floorDivClamped(floorf(fx1), S.sx) + 1);
     x0 = a;
     x1 = imax(a, c);
-}
-
-// coverageCount (tile_coverage.cpp:129-138).
-__device__ __forceinline__ uint32_t coverageCount(const Coverage& cv, const RowGeom& g, const BinShape& S) {
-    int r0, r1;
-    coverageRows(cv, S, r0, r1);
-    if (!cv.useEllipse) return uint32_t(imax(0, cv.bins.x1 - cv.bins.x0) * (r1 - r0));
-    uint32_t n = 0;
-    for (int r = r0; r < r1; ++r) {
-        int x0, x1;
-        coverageRowSpan(cv, g, r, S, x0, x1);
-        n += uint32_t(x1 - x0);
-    }
-    return n;
 }
 
 // Span hints: the coverage of a visible gaussian as its rows' runs, kept by the preprocess (which
