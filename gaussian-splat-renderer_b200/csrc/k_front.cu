@@ -306,8 +306,8 @@ __device__ __forceinline__ uint32_t preprocessOne(const FrontArgs& a, const DevC
 // the tensor cores for gaussians with a kept latent, the SH colour for the others.
 struct LearnedShared {
     DecoderWeights w;
-    __nv_bfloat16 stage[kFrontThreads / 32][32][16];
-    float out4[kFrontThreads / 32][32][4];
+    MlpRow stage[kFrontThreads / 32][32];
+    float4 out4[kFrontThreads / 32][32];
 };
 template <int COLOR>
 __device__ __forceinline__ void learnedColour(const FrontArgs& a, LearnedShared& sl, uint32_t i, size_t rec,

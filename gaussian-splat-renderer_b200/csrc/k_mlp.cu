@@ -545,17 +545,17 @@ __global__ void __launch_bounds__(128) encodeLatentsKernel(const float* __restri
 // The tensor-core decoder weights from the fp32 masters.
 __global__ void packDecoderKernel(const float* __restrict__ params, DecoderWeights* out) {
     using L = MlpLayout;
-    for (int e = threadIdx.x; e < 32 * 16; e += blockDim.x) {
-        const int n = e / 16, k = e % 16;
+    for (int e = threadIdx.x; e < 32 * (16 + kMlpPad); e += blockDim.x) {
+        const int n = e / (16 + kMlpPad), k = e % (16 + kMlpPad);
         out->w1[n][k] = __float2bfloat16_rn(k < kMlpIn ? params[L::kDecW1 + k * kMlpHidden + n] : 0.0f);
     }
-    for (int e = threadIdx.x; e < 32 * 32; e += blockDim.x) {
-        const int n = e / 32, k = e % 32;
-        out->w2[n][k] = __float2bfloat16_rn(params[L::kDecW2 + k * kMlpHidden + n]);
+    for (int e = threadIdx.x; e < 32 * (32 + kMlpPad); e += blockDim.x) {
+        const int n = e / (32 + kMlpPad), k = e % (32 + kMlpPad);
+        out->w2[n][k] = __float2bfloat16_rn(k < kMlpHidden ? params[L::kDecW2 + k * kMlpHidden + n] : 0.0f);
     }
-    for (int e = threadIdx.x; e < 8 * 32; e += blockDim.x) {
-        const int n = e / 32, k = e % 32;
-        out->w3[n][k] = __float2bfloat16_rn(n < kMlpOut ? params[L::kDecW3 + k * kMlpOut + n] : 0.0f);
+    for (int e = threadIdx.x; e < 8 * (32 + kMlpPad); e += blockDim.x) {
+        const int n = e / (32 + kMlpPad), k = e % (32 + kMlpPad);
+        out->w3[n][k] = __float2bfloat16_rn(n < kMlpOut && k < kMlpHidden ? params[L::kDecW3 + k * kMlpOut + n] : 0.0f);
     }
     for (int e = threadIdx.x; e < 32; e += blockDim.x) {
         out->b1[e] = params[L::kDecB1 + e];
@@ -579,8 +579,8 @@ struct GateArgs {
 constexpr int kGateWarps = 8;
 __global__ void __launch_bounds__(kGateWarps * 32) gateKernel(const __grid_constant__ GateArgs a) {
     __shared__ DecoderWeights W;
-    __shared__ __nv_bfloat16 stage[kGateWarps][32][16];
-    __shared__ float out4[kGateWarps][32][4];
+    __shared__ MlpRow stage[kGateWarps][32];
+    __shared__ float4 out4[kGateWarps][32];
     for (int e = threadIdx.x; e < int(sizeof(DecoderWeights) / 4); e += blockDim.x)
         reinterpret_cast<uint32_t*>(&W)[e] = reinterpret_cast<const uint32_t*>(a.decoder)[e];
     __syncthreads();

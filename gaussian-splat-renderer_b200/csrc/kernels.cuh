@@ -66,7 +66,7 @@ static_assert(sizeof(DevView) == 32, "DevView layout");
 // The learned colour stage's decoder for the tensor cores (mlp.cuh); the host needs its size and
 // the parameter count only.
 struct DecoderWeights;
-constexpr size_t kDecoderWeightsBytes = 32 * 16 * 2 + 32 * 32 * 2 + 8 * 32 * 2 + (32 + 32 + 8) * 4;
+constexpr size_t kDecoderWeightsBytes = 32 * 24 * 2 + 32 * 40 * 2 + 8 * 40 * 2 + (32 + 32 + 8) * 4;
 constexpr uint32_t kColorModelParams = 5195;
 constexpr size_t kColorTrainImageBytes = 24 * 1024;
 
