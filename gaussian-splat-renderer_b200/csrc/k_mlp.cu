@@ -602,7 +602,11 @@ __global__ void __launch_bounds__(kGateWarps * 32) gateKernel(const __grid_const
             for (int c = 0; c < 3; ++c) feat[kMlpLatent + c] = dir[c];
             float rgb[3], ref[3];
             mlpDecodeWarp(W, feat, stage[warp], out4[warp], rgb);
-            evalSH(int(a.degrees[g]), a.sh + size_t(g) * kEncIn, dir[0], dir[1], dir[2], ref);
+            alignas(16) float sh[kEncIn];  // the same words in every lane
+#pragma unroll
+            for (int k = 0; k < kEncIn / 4; ++k)
+                *reinterpret_cast<float4*>(&sh[4 * k]) = reinterpret_cast<const float4*>(a.sh + size_t(g) * kEncIn)[k];
+            evalSH(int(a.degrees[g]), sh, dir[0], dir[1], dir[2], ref);
             if (j < a.dirs) {
                 for (int c = 0; c < 3; ++c) {
                     const float d = fabsf(rgb[c] - ref[c]);

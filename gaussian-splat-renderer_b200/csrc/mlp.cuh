@@ -86,7 +86,8 @@ struct alignas(16) MlpRow {
 // memory. Rows of lanes that need no colour may hold anything.
 // Bound by shared memory where it is called back to back: unpadded rows, staged 16 bits at a time, took some
 // 400 wavefronts a call, twice what they take now (the gate over 64 directions of 559,000 gaussians
-// 1.5 -> 1.0 ms, the learned preprocess of 1.24 M at 1080p 152 -> 143 us).
+// 1.5 -> 1.0 ms, the learned preprocess of 1.24 M at 1080p 152 -> 143 us). A weight fragment is read once for both
+// halves of the warp's rows: 142 -> 136 us.
 __device__ __forceinline__ void mlpDecodeWarp(const DecoderWeights& W, const float (&feat)[kMlpIn],
                                               MlpRow* stage, float4* out4, float (&rgb)[3]) {
     const uint32_t lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
@@ -98,63 +99,76 @@ __device__ __forceinline__ void mlpDecodeWarp(const DecoderWeights& W, const flo
     stage[lane].q[0] = make_uint4(in[0], in[1], in[2], in[3]);
     stage[lane].q[1] = make_uint4(in[4], in[5], in[6], in[7]);
     __syncwarp();
+    uint32_t a[2][4];
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt) {
-        const int r0 = mt * 16 + g, r1 = r0 + 8;
-        uint32_t a[4];
-        a[0] = stage[r0].w[tig];
-        a[1] = stage[r1].w[tig];
-        a[2] = stage[r0].w[tig + 4];
-        a[3] = stage[r1].w[tig + 4];
-        // layer 1: 16 -> 32
-        float c1[4][4];
+        const MlpRow &r0 = stage[mt * 16 + g], &r1 = stage[mt * 16 + g + 8];
+        a[mt][0] = r0.w[tig];
+        a[mt][1] = r1.w[tig];
+        a[mt][2] = r0.w[tig + 4];
+        a[mt][3] = r1.w[tig + 4];
+    }
+    // the next layer's A fragments from this one's accumulators
+    auto activate = [](const float (&c)[2][4][4], uint32_t (&o)[2][2][4]) {
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            const int col = nt * 8 + tig * 2;
-            c1[nt][0] = W.b1[col]; c1[nt][1] = W.b1[col + 1]; c1[nt][2] = W.b1[col]; c1[nt][3] = W.b1[col + 1];
-            const int n = nt * 8 + g;
-            mmaBf16(c1[nt], a, *reinterpret_cast<const uint32_t*>(&W.w1[n][tig * 2]),
-                    *reinterpret_cast<const uint32_t*>(&W.w1[n][tig * 2 + 8]));
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int kb = 0; kb < 2; ++kb) {
+                o[mt][kb][0] = packBf16(fmaxf(c[mt][2 * kb][0], 0.0f), fmaxf(c[mt][2 * kb][1], 0.0f));
+                o[mt][kb][1] = packBf16(fmaxf(c[mt][2 * kb][2], 0.0f), fmaxf(c[mt][2 * kb][3], 0.0f));
+                o[mt][kb][2] = packBf16(fmaxf(c[mt][2 * kb + 1][0], 0.0f), fmaxf(c[mt][2 * kb + 1][1], 0.0f));
+                o[mt][kb][3] = packBf16(fmaxf(c[mt][2 * kb + 1][2], 0.0f), fmaxf(c[mt][2 * kb + 1][3], 0.0f));
+            }
+    };
+    // layer 1: 16 -> 32 (a weight fragment serves both halves of the warp's rows)
+    float c[2][4][4];
+    uint32_t h[2][2][4];
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+        const float2 b = *reinterpret_cast<const float2*>(&W.b1[nt * 8 + tig * 2]);
+        const int n = nt * 8 + g;
+        const uint32_t w0 = *reinterpret_cast<const uint32_t*>(&W.w1[n][tig * 2]);
+        const uint32_t w1 = *reinterpret_cast<const uint32_t*>(&W.w1[n][tig * 2 + 8]);
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+            c[mt][nt][0] = b.x; c[mt][nt][1] = b.y; c[mt][nt][2] = b.x; c[mt][nt][3] = b.y;
+            mmaBf16(c[mt][nt], a[mt], w0, w1);
         }
-        uint32_t a2[2][4];
+    }
+    activate(c, h);
+    // layer 2: 32 -> 32
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+        const float2 b = *reinterpret_cast<const float2*>(&W.b2[nt * 8 + tig * 2]);
+        const int n = nt * 8 + g;
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+            c[mt][nt][0] = b.x; c[mt][nt][1] = b.y; c[mt][nt][2] = b.x; c[mt][nt][3] = b.y;
+        }
 #pragma unroll
         for (int kb = 0; kb < 2; ++kb) {
-            a2[kb][0] = packBf16(fmaxf(c1[2 * kb][0], 0.0f), fmaxf(c1[2 * kb][1], 0.0f));
-            a2[kb][1] = packBf16(fmaxf(c1[2 * kb][2], 0.0f), fmaxf(c1[2 * kb][3], 0.0f));
-            a2[kb][2] = packBf16(fmaxf(c1[2 * kb + 1][0], 0.0f), fmaxf(c1[2 * kb + 1][1], 0.0f));
-            a2[kb][3] = packBf16(fmaxf(c1[2 * kb + 1][2], 0.0f), fmaxf(c1[2 * kb + 1][3], 0.0f));
+            const uint32_t w0 = *reinterpret_cast<const uint32_t*>(&W.w2[n][kb * 16 + tig * 2]);
+            const uint32_t w1 = *reinterpret_cast<const uint32_t*>(&W.w2[n][kb * 16 + tig * 2 + 8]);
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) mmaBf16(c[mt][nt], h[mt][kb], w0, w1);
         }
-        // layer 2: 32 -> 32
-        float c2[4][4];
+    }
+    activate(c, h);
+    // layer 3: 32 -> 8 (3 used)
+    const float2 b3 = *reinterpret_cast<const float2*>(&W.b3[tig * 2]);
+    float c3[2][4] = {{b3.x, b3.y, b3.x, b3.y}, {b3.x, b3.y, b3.x, b3.y}};
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            const int col = nt * 8 + tig * 2;
-            c2[nt][0] = W.b2[col]; c2[nt][1] = W.b2[col + 1]; c2[nt][2] = W.b2[col]; c2[nt][3] = W.b2[col + 1];
-            const int n = nt * 8 + g;
+    for (int kb = 0; kb < 2; ++kb) {
+        const uint32_t w0 = *reinterpret_cast<const uint32_t*>(&W.w3[g][kb * 16 + tig * 2]);
+        const uint32_t w1 = *reinterpret_cast<const uint32_t*>(&W.w3[g][kb * 16 + tig * 2 + 8]);
 #pragma unroll
-            for (int kb = 0; kb < 2; ++kb)
-                mmaBf16(c2[nt], a2[kb], *reinterpret_cast<const uint32_t*>(&W.w2[n][kb * 16 + tig * 2]),
-                        *reinterpret_cast<const uint32_t*>(&W.w2[n][kb * 16 + tig * 2 + 8]));
-        }
-        uint32_t a3[2][4];
+        for (int mt = 0; mt < 2; ++mt) mmaBf16(c3[mt], h[mt][kb], w0, w1);
+    }
+    if (tig < 2) {
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb) {
-            a3[kb][0] = packBf16(fmaxf(c2[2 * kb][0], 0.0f), fmaxf(c2[2 * kb][1], 0.0f));
-            a3[kb][1] = packBf16(fmaxf(c2[2 * kb][2], 0.0f), fmaxf(c2[2 * kb][3], 0.0f));
-            a3[kb][2] = packBf16(fmaxf(c2[2 * kb + 1][0], 0.0f), fmaxf(c2[2 * kb + 1][1], 0.0f));
-            a3[kb][3] = packBf16(fmaxf(c2[2 * kb + 1][2], 0.0f), fmaxf(c2[2 * kb + 1][3], 0.0f));
-        }
-        // layer 3: 32 -> 8 (3 used)
-        float c3[4];
-        const int col = tig * 2;
-        c3[0] = W.b3[col]; c3[1] = W.b3[col + 1]; c3[2] = W.b3[col]; c3[3] = W.b3[col + 1];
-#pragma unroll
-        for (int kb = 0; kb < 2; ++kb)
-            mmaBf16(c3, a3[kb], *reinterpret_cast<const uint32_t*>(&W.w3[g][kb * 16 + tig * 2]),
-                    *reinterpret_cast<const uint32_t*>(&W.w3[g][kb * 16 + tig * 2 + 8]));
-        if (tig < 2) {
-            reinterpret_cast<float2*>(&out4[r0])[tig] = make_float2(c3[0], c3[1]);
-            reinterpret_cast<float2*>(&out4[r1])[tig] = make_float2(c3[2], c3[3]);
+        for (int mt = 0; mt < 2; ++mt) {
+            reinterpret_cast<float2*>(&out4[mt * 16 + g])[tig] = make_float2(c3[mt][0], c3[mt][1]);
+            reinterpret_cast<float2*>(&out4[mt * 16 + g + 8])[tig] = make_float2(c3[mt][2], c3[mt][3]);
         }
     }
     __syncwarp();
