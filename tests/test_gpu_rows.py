@@ -59,7 +59,7 @@ def test_forms(gpu, bounds, splat, count):
 @pytest.mark.parametrize("count", [300, 40_000])
 def test_tall_splats_spill(gpu, count):
     """Vertical needles over all 68 tile rows: 300 fill a block's own part of the spilled runs, 40,000
-    need 2.7 M runs where the frame has 1.1 M, so most are computed again from their ellipses."""
+    need 2.7 M runs where the frame has 0.2 M, so most are computed again from their ellipses."""
     scene = tile_raster_scene(count, seed=3)
     n = np.arange(count)
     scene.pos_alpha[:, :3] = np.stack([(n % 997) / 997.0 * 9.0 - 4.5, np.zeros(count), (n % 31) * 0.01], 1)
