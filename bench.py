@@ -333,15 +333,16 @@ PASS_NAMES = {"preprocess": "reset + preprocess (depth keys)", "depth sort": "de
               "scan + emission": "scan + duplicate (depth order)", "tile sort": "tile sort (total)",
               "ranges": "tile ranges"}
 
-# DRAM bytes of the same passes (preprocess to ranges) for one frame of plain_1080p, from one
+# DRAM bytes of the same passes (preprocess to the list) for one frame of plain_1080p, from one
 # ncu capture of this build (dram__bytes_read.sum + dram__bytes_write.sum: preprocess, depth
-# sort histogram and its 3 active passes, scan, emission, tile sort histogram and 2 passes,
-# ranges); the bench cannot read the counters itself
-TRAFFIC_PLAIN_1080P_CAPTURE = (315.3 + 70.7 + 10.0 + 3 * 10.0 + 14.9 + 48.8 + 3.2 + 41.5 + 41.7 + 41.6 + 41.5) * 1e6
-# the same for one batched frame of 8 views (preprocess, depth sort histogram and its 3 active
-# passes, scan, emission, tile sort histogram and 2 passes, ranges)
-TRAFFIC_BATCHED_1080P_CAPTURE: dict = {8: (471.2 + 750.4 + 79.5 + 3 * 79.4 + 90.2 + 135.7 + 676.3 + 332.4 +
-                                           (332.2 + 291.0) + (332.2 + 291.3) + 332.8) * 1e6}
+# sort histogram and its 3 active passes, row plan, row partition, row tiles); the bench cannot read
+# the counters itself
+TRAFFIC_PLAIN_1080P_CAPTURE = (316.4 + 72.7 + 10.0 + 3 * 9.9 + 0.1 + 45.0 + 1.8 + 27.0 + 6.3) * 1e6
+# the same for one batched frame of 8 and of 16 views
+TRAFFIC_BATCHED_1080P_CAPTURE: dict = {8: (472.7 + 753.3 + 79.4 + 0.1 + 3 * (79.4 + 30.5) + 0.1 + 327.4 + 169.9 +
+                                           191.1 + 136.1) * 1e6,
+                                       16: (652.6 + 1593.7 + 158.9 + 0.1 + 3 * (158.8 + 113.6) + 0.1 + 650.5 + 371.8 +
+                                            384.8 + 330.1) * 1e6}
 
 
 # ---- the CPU leg: the reference's renderer as the baseline and as the checker of the GPU's views
@@ -601,7 +602,7 @@ def roofline(passes: dict, ctl, fmt: str, n: int, tiles: int, peak: float, peak_
     kernels, tot_b, tot_ms = {}, 0.0, 0.0
     for k, nb in b.items():
         ms = passes.get(PASS_NAMES[k])
-        if not ms:
+        if not ms or not nb:  # (a row-wise list has no ranges pass)
             continue
         gbs = nb / (ms * 1e-3) / 1e9
         kernels[k] = {"bytes": int(nb), "ms": ms, "GB/s": round(gbs, 1), "frac": round(gbs / peak, 4)}
@@ -657,8 +658,8 @@ def render_issue(passes: dict, clocks: dict, instructions: float | None):
 
 # warp instructions (smsp__inst_executed.sum) of one 1080p view's render pass and preprocess,
 # from an ncu capture of this build (the plain profiling mode, two launches of each kernel)
-RENDER_WARP_INSTRUCTIONS_1080P = 209.69e6
-PREPROCESS_WARP_INSTRUCTIONS_1080P = 75.17e6
+RENDER_WARP_INSTRUCTIONS_1080P = 157.75e6
+PREPROCESS_WARP_INSTRUCTIONS_1080P = 74.32e6
 
 
 def issue_roofline(passes: dict, clocks: dict, views: int) -> dict | None:
