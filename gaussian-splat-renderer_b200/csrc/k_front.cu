@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(kFrontThreads, 4) preprocessKernel(const __gri
                 const uint32_t at = terms[(kRowTermWords + 2) * 32 + q], row = (who & 0xFFFFu) + k;
                 int x0, x1;
                 rowTermsSpan(t, int(row), bs, x0, x1);
-                const uint32_t tiles = uint32_t(x1 - x0), run = uint32_t(x0) | (uint32_t(x1) << 16);
+                const uint32_t tiles = uint32_t(x1 - x0), run = packRun(x0, x1);
                 atomicAdd(&terms[(kRowTermWords + 3) * 32 + q], tiles);
                 if (a.rowRecords && tiles) atomicAdd(&sRows[row & (kRowBins - 1u)], (1u << 20) | tiles);
                 const size_t r = warpRec + (who >> 16);

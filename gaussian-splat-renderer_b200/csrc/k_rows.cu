@@ -90,7 +90,7 @@ __device__ __noinline__ uint32_t ellipseRun(const FrontArgs& a, const DevView& v
     const Coverage cv = recordCoverage(a, vw, rec, g);
     int x0, x1;
     coverageRowSpan(cv, g, int(row), binShapeOf(a.binSize), x0, x1);
-    return uint32_t(x0) | (uint32_t(x1) << 16);
+    return packRun(x0, x1);
 }
 __device__ __noinline__ uint4 ellipseRows(const FrontArgs& a, const DevView& vw, size_t rec) {  // r0, rows, first run, rest
     RowGeom g;
@@ -98,7 +98,7 @@ __device__ __noinline__ uint4 ellipseRows(const FrontArgs& a, const DevView& vw,
     int r0, r1;
     coverageRows(cv, binShapeOf(a.binSize), r0, r1);
     return make_uint4(uint32_t(r0), uint32_t(r1 - r0),
-                      uint32_t(cv.bins.x0) | (uint32_t(imax(cv.bins.x0, cv.bins.x1)) << 16),
+                      packRun(cv.bins.x0, cv.bins.x1),
                       cv.useEllipse ? kRunsEllipse : kRunsSame);
 }
 
@@ -193,7 +193,8 @@ struct WarpPairs {
 };
 
 // fn(valid, row, run x0 | x1 << 16, gaussian) for the runs of the warp's 32 records in (record, row)
-// order, 32 at a time, all lanes together; terms = kTermWords x 32 words of the warp's shared memory.
+// order, 32 at a time, all lanes together (valid: not empty, and inside the view whatever the word holds);
+// terms = kTermWords x 32 words of the warp's shared memory.
 constexpr uint32_t kTermWords = 4 + kSpanRows;
 template <typename Fn>
 __device__ __forceinline__ void forWarpRuns(const FrontArgs& a, const DevView& vw, uint32_t view, size_t rec, const RecordRows& R,
@@ -227,7 +228,7 @@ __device__ __forceinline__ void forWarpRuns(const FrontArgs& a, const DevView& v
             else if (at == kRunsEllipse) run = ellipseRun(a, vw, owner, row);
             else run = a.spill[at + r];
         }
-        fn((run >> 16) > (run & 0xFFFFu) && row < kRowBins, row, run, gaussian);
+        fn((run >> 16) > (run & 0xFFFFu) && (run >> 16) <= vw.tilesX && row < vw.tilesY, row, run, gaussian);
     }
 }
 

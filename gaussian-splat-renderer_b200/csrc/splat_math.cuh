@@ -390,6 +390,11 @@ __device__ __forceinline__ bool isSpanHint(const float4& h) {
     return (__float_as_uint(h.x) & 0xFFC00000u) == kSpanMarker;
 }
 
+// A row's run of tiles [x0, x1) in one word, x0 | x1 << 16. An empty one is 0 wherever it lies: an ellipse
+// that is right of the image at this row has both ends at up to 131,072 (floorDivClamped), past the 16
+// bits, and a packed end would read as a run of the image's first tiles.
+__device__ __forceinline__ uint32_t packRun(int x0, int x1) { return x1 > x0 ? uint32_t(x0) | (uint32_t(x1) << 16) : 0u; }
+
 // What a row's run is computed from (coverageRowSpan's inputs), as a warp's lanes pass it around.
 struct RowTerms {
     float cx, cy, A, B, D, eyPad, eyRight0, At, pad;
