@@ -190,6 +190,7 @@ __device__ __forceinline__ void viewDirection(const float4& pa, const float (&ca
 struct ColourJob {
     uint32_t meta, degree;
     float dir[3];  // normalize(mean - camera position), glm::normalize's order
+    bool landed;   // staged SH: the wait for the copy (shColour's) did not expire
 };
 
 // Staged SH (soa scenes with 16 stored coefficients and no per-gaussian degree): at block start
@@ -235,11 +236,13 @@ __device__ __forceinline__ void issueShStage(const SceneArgs& s, uint32_t i0, ui
                  :: "r"(smemAddr(gShStage)), "l"(src), "r"(bytes), "r"(smemAddr(&gShBarrier)) : "memory");
 }
 
-// The plain colour: the gaussian's SH coefficients, evaluated in the view direction.
+// The plain colour: the gaussian's SH coefficients, evaluated in the view direction. Returns whether the
+// staged copy had landed.
 template <int COLOR>
-__device__ __forceinline__ void shColour(const FrontArgs& a, uint32_t i, const ColourJob& job, DevSplat& s) {
+__device__ __forceinline__ bool shColour(const FrontArgs& a, uint32_t i, const ColourJob& job, DevSplat& s) {
     float color[3];
-    if (COLOR == GSR_COLOR_SOA_F32 && a.shStaged && waitShStage(a.ctl, true)) {
+    const bool landed = COLOR == GSR_COLOR_SOA_F32 && a.shStaged && waitShStage(a.ctl, true);
+    if (landed) {
         // straight from the staged copy: the coefficients are read as the bands need them, with
         // no 48-register array (evalSH reads the first (degree + 1)^2 triplets)
         evalSH(int(job.degree), reinterpret_cast<const float*>(gShStage + threadIdx.x * 12), job.dir[0], job.dir[1],
@@ -252,6 +255,7 @@ __device__ __forceinline__ void shColour(const FrontArgs& a, uint32_t i, const C
     s.r = color[0];
     s.g = color[1];
     s.b = color[2];
+    return landed;
 }
 
 // preprocessGaussian (splat_math.cpp:153-193) with the GPU culls of splat_preprocess.comp.
@@ -286,7 +290,7 @@ __device__ __forceinline__ uint32_t preprocessOne(const FrontArgs& a, const DevC
     job.meta = meta;
     job.degree = uint32_t(a.evalDegree) < gdeg ? uint32_t(a.evalDegree) : gdeg;
     viewDirection(pa, cam.pos, job.dir);
-    if (!LEARNED) shColour<COLOR>(a, i, job, s);
+    if (!LEARNED) job.landed = shColour<COLOR>(a, i, job, s);
     s.conicA = conic[0];
     s.conicB = conic[1];
     s.conicC = conic[2];
@@ -515,9 +519,10 @@ __global__ void __launch_bounds__(kFrontThreads, 4) preprocessKernel(const __gri
     // the longest of 32 has eight or more, so a lane walking its own rows left most lanes idle (preprocess
     // of 1.24 M gaussians 141 -> 125 us, of eight views 890 -> 788, of 6 M at 4K 531 -> 460). The terms go
     // through shared memory, under the splat's place among those with rows; the SH staging area is free once
-    // the warp's colours are done.
-    if (a.bounds != kBoundsRect && __any_sync(0xFFFFFFFFu, rows != 0)) {
-        if (staged && !shStageReady()) waitShStage(a.ctl, false);  // (a forced expiry reads on before the copy has landed)
+    // the copy into it has landed and the warp's colours are done. If the wait for it expires, the copy may
+    // land over the terms (which say where runs are stored), so the warp's splats get no tiles.
+    if (a.bounds != kBoundsRect && __any_sync(0xFFFFFFFFu, rows != 0) &&
+        __all_sync(0xFFFFFFFFu, !staged || rows == 0 || job.landed)) {
         uint32_t* terms = reinterpret_cast<uint32_t*>(gShStage) + (tid >> 5) * (staged ? 32u * 48u : 32u * kRunWords);
         const uint32_t has = __ballot_sync(0xFFFFFFFFu, rows != 0), belowLane = (1u << lane) - 1u;
         uint32_t end = rows;
