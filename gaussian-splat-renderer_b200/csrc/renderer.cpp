@@ -823,6 +823,7 @@ struct GsrRenderer {
     // Per-gaussian arrays and the frame slots' camera copies for `v` views (grown, never shrunk).
     int ensureViews(uint32_t v) {
         if (v <= allocViews) return GSR_OK;
+        allocViews = 0;  // until all of them are there
         const size_t n = size_t(scene.count) * v;
         if (settings.render_splat == GSR_RENDER_SPLAT_FULL) {
             GSR_CUDA(splats.alloc(n * 48));
@@ -862,8 +863,8 @@ struct GsrRenderer {
         return GSR_OK;
     }
 
-    // onRenderTargetsChanged for the views' sizes: the per-tile and image buffers of the frame's
-    // tiles and pixels over all views, and the list when the key width changes.
+    // onRenderTargetsChanged for the views' sizes. A layout that could not be completed is none: the next
+    // call sets one up from the start, with a list of its own.
     int setLayout(const uint32_t* w, const uint32_t* h, uint32_t v) {
         if (v == 0 || v > GSR_MAX_VIEWS) return fail(GSR_ERROR_INVALID_ARGUMENT, "views %u (1..%u)", v, GSR_MAX_VIEWS);
         if (copyStream) GSR_CUDA(cudaStreamSynchronize(copyStream));  // copies still reading the old images
@@ -882,6 +883,17 @@ struct GsrRenderer {
         if (same) return GSR_OK;
         if (tiles >= (1ull << 31)) return fail(GSR_ERROR_INVALID_ARGUMENT, "%llu tiles in one frame", (unsigned long long)tiles);
         GSR_CUDA(cudaDeviceSynchronize());  // the reference calls onRenderTargetsChanged with the GPU idle
+        const int rc = layOut(w, h, v, tiles, pixels);
+        if (rc) {
+            views.clear();
+            passesUpper = 0;
+        }
+        return rc;
+    }
+
+    // The per-tile and image buffers of the frame's tiles and pixels over all views, and the list when the
+    // key width changes.
+    int layOut(const uint32_t* w, const uint32_t* h, uint32_t v, uint64_t tiles, uint64_t pixels) {
         int rc = ensureViews(v);
         if (rc) return rc;
         views.assign(v, GsrViewLayout{});
@@ -1746,7 +1758,7 @@ int gsr_read_control(GsrRenderer* r, GsrControl* out) {
 
 int gsr_read_list(GsrRenderer* r, uint32_t* keysLo, uint32_t* keysHi, uint32_t* values, uint32_t n, uint32_t* rangesOut,
                   uint32_t rangesWords) {
-    if (!r || !r->list) return fail(GSR_ERROR_INVALID_ARGUMENT, "no list");
+    if (!r || !r->list || r->views.empty()) return fail(GSR_ERROR_INVALID_ARGUMENT, "no list");
     GSR_CUDA(cudaDeviceSynchronize());
     GsrControl c;
     GSR_CUDA(cudaMemcpy(&c, &r->control.as<DeviceControl>()->c, sizeof(c), cudaMemcpyDeviceToHost));
