@@ -361,13 +361,18 @@ cudaError_t uploadHost(const std::vector<Upload>& parts) {
     std::atomic<size_t> next{0};
     std::atomic<int> failed{int(cudaSuccess)};
     auto work = [&](unsigned id) {
-        cudaError_t e = cudaSetDevice(dev);
         cudaStream_t s = nullptr;
         cudaEvent_t free[2] = {nullptr, nullptr};
-        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-        for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&free[k], cudaEventDisableTiming);
+        bool ready = cudaSetDevice(dev) == cudaSuccess && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
+        if (!ready) s = nullptr;
+        for (int k = 0; k < 2 && ready; ++k) {
+            ready = cudaEventCreateWithFlags(&free[k], cudaEventDisableTiming) == cudaSuccess;
+            if (!ready) free[k] = nullptr;
+        }
+        if (!ready) cudaGetLastError();  // the other threads take the pieces, or the copies after them
+        cudaError_t e = cudaSuccess;
         unsigned char* slot = static_cast<unsigned char*>(g_stager.slots) + size_t(id) * 2 * Stager::kPiece;
-        for (unsigned n = 0; e == cudaSuccess && failed.load() == int(cudaSuccess); ++n) {
+        for (unsigned n = 0; ready && e == cudaSuccess && failed.load() == int(cudaSuccess); ++n) {
             const size_t p = next.fetch_add(1);
             if (p >= pieces.size()) break;
             const unsigned k = n & 1u;
@@ -403,7 +408,9 @@ cudaError_t uploadHost(const std::vector<Upload>& parts) {
     }
     work(0);
     for (std::thread& t : threads) t.join();
-    return cudaError_t(failed.load());
+    if (failed.load() != int(cudaSuccess) || next.load() >= pieces.size()) return cudaError_t(failed.load());
+    pieces.erase(pieces.begin(), pieces.begin() + std::ptrdiff_t(next.load()));  // no thread could take them
+    return uploadPlain(pieces);
 }
 }  // namespace
 
