@@ -342,9 +342,11 @@ cudaError_t uploadPlain(const std::vector<Upload>& parts) {
 cudaError_t uploadHost(const std::vector<Upload>& parts) {
     size_t total = 0;
     for (const Upload& u : parts) total += u.bytes;
-    cudaPointerAttributes at{};
-    const bool locked = !parts.empty() && cudaPointerGetAttributes(&at, parts.back().src) == cudaSuccess &&
-                        at.type != cudaMemoryTypeUnregistered;
+    bool locked = false;  // any of them: a plain copy waits for the work that may still be filling it
+    for (const Upload& u : parts) {
+        cudaPointerAttributes at{};
+        locked |= cudaPointerGetAttributes(&at, u.src) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
+    }
     if (locked || total < Stager::kMin) return uploadPlain(parts);
     std::unique_lock<std::mutex> lock(g_stager.use, std::try_to_lock);
     int dev = 0;

@@ -1,5 +1,6 @@
 """The threaded scene upload when one of its threads, or all of them, cannot set up a stream or an event,
-or the slots cannot be page-locked: the scene holds the arrays all the same (a failed transfer is reported)."""
+or the slots cannot be page-locked: the scene holds the arrays all the same (a failed transfer is reported).
+An upload with any page-locked array is a plain copy, in the order of the work before it."""
 import numpy as np
 import pytest
 
@@ -43,3 +44,13 @@ def test_failed_transfer(fake, host, nth):  # noqa: F811
         gsr_b200.GpuScene(host)
     fake.fake_fail(b"cudaMemcpyAsync", 0)
     _check(host)
+
+
+@pytest.mark.parametrize("array", ["pos_alpha", "scales", "rotations", "sh"])
+def test_a_page_locked_array(fake, host, array):  # noqa: F811
+    a = getattr(host, array)
+    fake.fake_page_locked(a.ctypes.data, a.nbytes)
+    before = fake.fake_calls(b"cudaMemcpyAsync"), fake.fake_calls(b"cudaHostAlloc")
+    _check(host)
+    assert before == (fake.fake_calls(b"cudaMemcpyAsync"), fake.fake_calls(b"cudaHostAlloc"))
+    fake.fake_page_locked(a.ctypes.data, 0)
