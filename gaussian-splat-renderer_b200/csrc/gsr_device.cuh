@@ -62,7 +62,9 @@ __device__ __forceinline__ void reportTimeout(DeviceControl* ctl, uint32_t where
 // Decoupled look-back (single-pass chained scan, Merrill & Garland 2016) of one tile's
 // exclusive prefix, done by one full warp: lane j inspects predecessor (tile - 1 - j) so a
 // window of 32 predecessors is read per step. Returns the sum of the values of all tiles
-// before `tile`. Waits are bounded by kSpinLimit (then reportTimeout and a partial sum).
+// before `tile`. Waits are bounded by kSpinLimit (then reportTimeout and a partial sum). The sum is modulo
+// 2^32, or with SATURATE 2^32 - 1 from there on.
+template <bool SATURATE = false>
 __device__ __forceinline__ uint32_t warpLookback(const uint64_t* status, int tile, uint32_t epoch,
                                                  DeviceControl* ctl, uint32_t where) {
     const int lane = threadIdx.x & 31;
@@ -89,7 +91,13 @@ __device__ __forceinline__ uint32_t warpLookback(const uint64_t* status, int til
             const int first = __ffs(incl) - 1;
             if (lane > first) v = 0;
         }
-        exclusive += __reduce_add_sync(0xFFFFFFFFu, v);
+        if constexpr (SATURATE) {
+            const uint64_t high = __reduce_add_sync(0xFFFFFFFFu, v >> 16), low = __reduce_add_sync(0xFFFFFFFFu, v & 0xFFFFu);
+            const uint64_t sum = exclusive + (high << 16) + low;
+            exclusive = sum < 0xFFFFFFFFull ? uint32_t(sum) : 0xFFFFFFFFu;
+        } else {
+            exclusive += __reduce_add_sync(0xFFFFFFFFu, v);
+        }
         if (incl) break;
         base -= 32;
     }

@@ -344,13 +344,14 @@ __global__ void __launch_bounds__(kRowThreads) rowPlanKernel(const __grid_consta
             n[j] = some[j] ? a.tileCounts[rec[j]] : 0u;
             mine += n[j];
         }
-        uint64_t total;
-        uint32_t at = uint32_t(blockScan64(mine, sWarp, &total));
+        // (a prefix past 2^32 - 1 stays there: it is past every capacity)
+        uint64_t total, at = blockScan64(mine, sWarp, &total);
         if (warp == 0) {
             if (lane == 0) stRelaxed(&a.scanStatus[t], packStatus(epoch, t == 0 ? kFlagInclusive : kFlagAggregate, uint32_t(total)));
-            const uint32_t before = t ? warpLookback(a.scanStatus, int(t), epoch, ctl, kWaitScan) : 0u;
+            const uint32_t before = t ? warpLookback<true>(a.scanStatus, int(t), epoch, ctl, kWaitScan) : 0u;
+            const uint64_t through = before + total;
             if (lane == 0) {
-                if (t) stRelaxed(&a.scanStatus[t], packStatus(epoch, kFlagInclusive, before + uint32_t(total)));
+                if (t) stRelaxed(&a.scanStatus[t], packStatus(epoch, kFlagInclusive, through < 0xFFFFFFFFull ? uint32_t(through) : 0xFFFFFFFFu));
                 sExclusive = before;
             }
         }
@@ -360,8 +361,9 @@ __global__ void __launch_bounds__(kRowThreads) rowPlanKernel(const __grid_consta
         RecordRows R[kRowSteps];
 #pragma unroll
         for (uint32_t j = 0; j < kRowSteps; ++j) {
-            kept[j] = at < a.capacity ? (n[j] < a.capacity - at ? n[j] : a.capacity - at) : 0u;
-            if (n[j] && at < a.capacity && a.capacity - at <= n[j]) {  // one record of the frame
+            const uint32_t room = at < a.capacity ? a.capacity - uint32_t(at) : 0u;
+            kept[j] = n[j] < room ? n[j] : room;
+            if (room && n[j] >= room) {  // one record of the frame
                 ctl->rowCutSlot = base + j;
                 ctl->rowCutTiles = kept[j];
             }

@@ -1,0 +1,52 @@
+"""Frames of more than 2^32 tiles: the row-wise list is still the full one cut at its capacity in (depth,
+gaussian, tile) order. The splats are placed so that the whole list is known: their depths order like their
+indices."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(count, x, scale, alpha):
+    from gsr_b200 import scenes
+
+    pos = np.zeros((count, 4), np.float32)
+    pos[:, 0] = x
+    pos[:, 2] = np.linspace(2.0, -2.0, count)  # the camera looks along -z from z = 6
+    pos[:, 3] = alpha
+    scales = np.zeros((count, 4), np.float32)
+    scales[:, :3] = scale
+    rotations = np.zeros((count, 4), np.float32)
+    rotations[:, 0] = 1.0
+    return scenes.Scene(pos, scales, rotations, np.zeros(count * 3, np.float32), 0)
+
+
+def _frame(gpu, scene, width, height, bounds):
+    from gsr_b200 import scenes
+
+    gs = gpu.GpuScene(scene)
+    r = gpu.Renderer(gs, gpu.Settings(adaptive_list=False, budget_mb=4, bounds=bounds))
+    r.render(scenes.viewer_camera((0.0, 0.0, 6.0), (0.0, 0.0, 0.0), width, height, 60.0))
+    _, hi, val, ranges, ctl = r.read_back()
+    cap = r.capacity()[0]
+    assert ctl.status == 0 and ctl.ext_pad[0] > 0, ctl.as_dict()
+    assert ctl.duplicates == 0xFFFFFFFF and ctl.entries == cap and ctl.overflow == 0xFFFFFFFF - cap
+    r.close()
+    gs.close()
+    return hi, val, ranges, cap
+
+
+def _every_tile(gpu, count, width, height):
+    """Splats that cover every tile: the list holds the first ones in every tile, the last of them in the
+    tiles that are left."""
+    hi, val, ranges, cap = _frame(gpu, _scene(count, 0.0, 60.0, 0.5), width, height, "rect")
+    tiles = (width // 16) * (height // 16)
+    of_tile = cap // tiles + (np.arange(tiles) < cap % tiles)
+    end = np.cumsum(of_tile)
+    np.testing.assert_array_equal(ranges, np.stack([end - of_tile, end], 1))
+    np.testing.assert_array_equal(hi, np.repeat(np.arange(tiles), of_tile))
+    np.testing.assert_array_equal(val, np.arange(cap) - np.repeat(end - of_tile, of_tile))
+
+
+def test_prefix_past_32_bits(gpu):
+    _every_tile(gpu, 4_300_000, 512, 512)  # 1,024 tiles each
