@@ -40,7 +40,7 @@ struct DeviceControl {
     uint32_t rowCutTiles;       // ... and the tiles of it that are kept
     uint32_t forceTimeout;      // test hook: look-back waits see no predecessor for this many spins
     uint32_t spillCursor;       // row-wise list: the spilled runs taken so far
-    uint32_t pad[2];
+    unsigned long long rowTiles;  // ... and the frame's tiles (FrontArgs::rowTilesWide)
 };
 
 // Items of one block of the exclusive scan (scanKernel: 256 threads x kScanItems); the scan's

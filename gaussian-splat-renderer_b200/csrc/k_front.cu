@@ -414,7 +414,8 @@ __global__ void __launch_bounds__(kFrontThreads, 4) preprocessKernel(const __gri
     __shared__ uint32_t sCull[kCullReasonCount];
     __shared__ uint32_t sDepthMin, sDepthMax;
     __shared__ uint32_t sRows[kRowBins];  // row-wise lists: a row's entries << 20 | tiles, of this block
-    __shared__ uint32_t sSpilled;         // ... and the spilled runs it has taken of its own part
+    __shared__ uint32_t sSpilled;         // ... the spilled runs it has taken of its own part
+    __shared__ uint32_t sTiles;           // ... and its tiles (131,072 a splat at most)
     const uint32_t tid = threadIdx.x, lane = tid & 31;
     gridWait();
     // the views vary fastest along the grid: the blocks of one gaussian range for every view run
@@ -423,8 +424,9 @@ __global__ void __launch_bounds__(kFrontThreads, 4) preprocessKernel(const __gri
     if (tid < kCullReasonCount) sCull[tid] = 0;
     static_assert(kRowBins == kFrontThreads && kFrontThreads * kRowMaxTilesX < (1u << 20), "a block's row counts");
     if (a.rowRecords) sRows[tid] = 0;
-    if (tid == 0) sSpilled = 0;
     if (tid == 0) {
+        sSpilled = 0;
+        sTiles = 0;
         sDepthMin = 0xFFFFFFFFu;
         sDepthMax = 0;
     }
@@ -586,6 +588,10 @@ __global__ void __launch_bounds__(kFrontThreads, 4) preprocessKernel(const __gri
             a.depthKeys[0][rec] = (a.depthViewShift ? uint64_t(view) << a.depthViewShift : 0ull) |
                                   (uint64_t(count ? __float_as_uint(s.depth) : 0xFFFFFFFFu) << a.recordBits) | rec;
     }
+    if (a.rowTilesWide) {
+        const uint32_t n = __reduce_add_sync(0xFFFFFFFFu, count);
+        if (lane == 0 && n) atomicAdd(&sTiles, n);
+    }
 #pragma unroll
     for (uint32_t r = 0; r < kCullReasonCount; ++r) {
         const uint32_t n = __popc(__ballot_sync(0xFFFFFFFFu, reason == r));
@@ -606,6 +612,7 @@ __global__ void __launch_bounds__(kFrontThreads, 4) preprocessKernel(const __gri
     if (a.rowRecords && sRows[tid])
         atomicAdd(&a.rowHist[size_t(view) * kRowBins + tid],
                   (static_cast<unsigned long long>(sRows[tid] >> 20) << 32) | (sRows[tid] & 0xFFFFFu));
+    if (a.rowTilesWide && tid == 0 && sTiles) atomicAdd(&a.ctl->rowTiles, static_cast<unsigned long long>(sTiles));
     if (tid < kCullReasonCount && sCull[tid]) atomicAdd(&a.ctl->c.cull_counts[tid], sCull[tid]);
     if (tid == 0 && sDepthMin <= sDepthMax) {
         atomicMin(&a.ctl->c.depth_min_bits, sDepthMin);
@@ -844,6 +851,7 @@ __global__ void frameBeginKernel(DeviceControl* ctl, uint32_t count, uint32_t ca
         ctl->histDone[0] = 0;
         ctl->histDone[1] = 0;
         ctl->spillCursor = 0;
+        ctl->rowTiles = 0;
         ctl->forceTimeout = forceTimeout;
     }
 }

@@ -298,11 +298,14 @@ __global__ void __launch_bounds__(kRowThreads) rowPlanKernel(const __grid_consta
     gridWait();
     DeviceControl* ctl = a.ctl;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // every block adds up the frame's tiles (the low words: their sum fits, M < 2^32)
-    uint64_t sum = 0, all;
+    // every block adds up the frame's tiles from the rows' low words, unless one of them may have gone past
+    // 2^32 and carried into its entries (which are not read then: a full list is planned from its kept records)
+    uint64_t sum = 0, all = ctl->rowTiles;
+    if (!a.rowTilesWide) {
 #pragma unroll 8
-    for (uint32_t j = tid; j < a.viewCount * kRowBins; j += kRowThreads) sum += __ldcg(&a.rowHist[j]) & 0xFFFFFFFFull;
-    blockScan64(sum, sWarp, &all);
+        for (uint32_t j = tid; j < a.viewCount * kRowBins; j += kRowThreads) sum += __ldcg(&a.rowHist[j]) & 0xFFFFFFFFull;
+        blockScan64(sum, sWarp, &all);
+    }
     const uint32_t tiles = uint32_t(all < 0xFFFFFFFFull ? all : 0xFFFFFFFFull);
     const bool full = tiles > a.capacity;
     if (blockIdx.x == 0 && tid == 0) {

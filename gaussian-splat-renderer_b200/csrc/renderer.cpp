@@ -1174,6 +1174,7 @@ struct GsrRenderer {
             fa.depthViewShift = viewBits ? fa.recordBits + 32u : 0u;
             if (rowWise) {
                 fa.rowRecords = 1;
+                fa.rowTilesWide = uint64_t(scene.count) * maxTilesX >= (1ull << 32) ? 1u : 0u;
                 fa.rowsPerView = maxTilesY;
                 fa.buckets = reinterpret_cast<const uint32_t*>(viewsDevice.as<DevView>() + viewCount);
                 fa.bucketCount = uint32_t(totalRows);

@@ -50,3 +50,7 @@ def _every_tile(gpu, count, width, height):
 
 def test_prefix_past_32_bits(gpu):
     _every_tile(gpu, 4_300_000, 512, 512)  # 1,024 tiles each
+
+
+def test_a_row_past_32_bits(gpu):
+    _every_tile(gpu, 2 ** 23, 8192, 688)  # 512 tiles of each of the 43 rows: 2^32 a row
