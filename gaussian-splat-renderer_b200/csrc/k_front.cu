@@ -497,7 +497,9 @@ __global__ void __launch_bounds__(kFrontThreads, 4) preprocessKernel(const __gri
                     if (own + n <= kSpillPerBlock) {
                         runsAt = blockIdx.x * kSpillPerBlock + own;
                     } else {  // the block's part is full: from the frame's common part
-                        const uint32_t at = atomicAdd(&a.ctl->spillCursor, n), common = a.spillCapacity - gridDim.x * kSpillPerBlock;
+                        // (not asked once it is taken, so that the cursor, 256 a splat, stays below 2^32)
+                        const uint32_t common = a.spillCapacity - gridDim.x * kSpillPerBlock;
+                        const uint32_t at = __ldcg(&a.ctl->spillCursor) <= common ? atomicAdd(&a.ctl->spillCursor, n) : common;
                         if (at <= common && n <= common - at) runsAt = gridDim.x * kSpillPerBlock + at;
                     }
                 }
