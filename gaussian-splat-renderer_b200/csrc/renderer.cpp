@@ -595,12 +595,19 @@ struct GsrRenderer {
     // records leave the chip idle. Frames, row by row against sorted (us): 133,000 records a row
     // (4 M at 640 x 480) 743 against 782, 155,000 (1.24 M at 1280 x 128) 466 against 495, 250,000
     // (4 M at 256 x 256) 684 against 654.
+    // Nor many rows of few records: a row costs its eight blocks whatever it holds (about 0.08 us). Over
+    // 1,000 to 200,000 gaussians in 2 to 256 views, beyond 384 rows: 1,000 in 256 views of 256 x 256 842
+    // against 445, 15,000 in 64 555 against 480, 30,000 in 64 888 against 831, 45,000 in 48 of 1280 x 720
+    // 2,370 against 2,381; up to 384 rows 0.76 to 1.14 of the sorted list. The line lies lower with
+    // small tiles, of which a splat has more to sort (30,000 in 8 views of 1280 x 720, 8-px tiles: 491
+    // against 513), and higher with 32 x 8 ones (60,000: 625 against 606).
     bool rowWiseFits(uint32_t v) const {
+        const uint32_t few = settings.tile_size == 8 ? 20000u : settings.tile_size == 16 ? 40000u : 65000u;
         return binning() && maxTilesY <= kRowBins && maxTilesX <= kRowMaxTilesX &&
-               uint64_t(scene.count) * v <= kRowMaxRecords * totalRows;
+               uint64_t(scene.count) * v <= kRowMaxRecords * totalRows && (totalRows <= kRowFewRows || scene.count > few);
     }
     uint64_t totalRows = 0;
-    static constexpr uint64_t kRowMaxRecords = 196608;
+    static constexpr uint64_t kRowMaxRecords = 196608, kRowFewRows = 384;
     uint32_t rowHistWords() const { return allocViews * kRowBins * 2 * 2; }
     uint32_t rowStatusVec4s(uint32_t v) const {
         const uint64_t tile = rowPartitionTile(uint64_t(scene.count) * v);
