@@ -583,7 +583,9 @@ struct GsrRenderer {
     // A row-wise list's work for allocViews views: the look-back words of the partition, the buckets, the
     // runs of splats of many rows (each preprocess block's own, and a common part of four a record, at most
     // a million: a flat million, 4 MB, made scene and renderer of 10,000 gaussians 1.6 instead of 0.9 ms).
+    // Given back while the layout's list is sorted.
     DevBuf rowWork;
+    size_t rowWorkBytes(size_t v) const { return rowStatusBytes(v) + v * kRowBins * 16 + spillRuns(v) * 4; }
     size_t rowStatusBytes(size_t v) const { return v * ((size_t(scene.count) + kRowPartTile - 1) / kRowPartTile) * kRowBins * 4; }
     size_t spillRuns(size_t v) const {
         return v * ((size_t(scene.count) + 255) / 256) * kSpillPerBlock + std::min<size_t>(v * scene.count * 4, 1u << 20);
@@ -863,7 +865,7 @@ struct GsrRenderer {
             GSR_CUDA(cudaMemset(depthStatus.p, 0, depthStatus.bytes));
             GSR_CUDA(depthRuns.alloc(size_t(v) * kRowBins * 2 * 2 * 4 + size_t(depthRunWords(v)) * 2 * 4));
             GSR_CUDA(cudaMemset(depthRuns.p, 0, depthRuns.bytes));
-            GSR_CUDA(rowWork.alloc(rowStatusBytes(v) + size_t(v) * kRowBins * 16 + spillRuns(v) * 4));
+            GSR_CUDA(rowWork.alloc(rowWorkBytes(v)));
         }
         GSR_CUDA(tileCounts.alloc(n * 4));
         offsets.release();  // (sortedListReady)
@@ -941,6 +943,8 @@ struct GsrRenderer {
         totalTiles = uint32_t(tiles);
         totalPixels = pixels;
         rowWise = rowWiseFits(v);
+        if (!rowWise) rowWork.release();
+        else if (!rowWork.p) GSR_CUDA(rowWork.alloc(rowWorkBytes(allocViews)));
         width = views[0].width;
         height = views[0].height;
         tilesX = views[0].tiles_x;

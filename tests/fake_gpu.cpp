@@ -16,7 +16,7 @@
 namespace {
 std::mutex g_mutex;
 std::map<std::string, int> g_calls, g_failFrom;
-std::map<const void*, size_t> g_locked;
+std::map<const void*, size_t> g_locked, g_live;
 std::atomic<int> g_nullLaunches{0};
 
 cudaError_t called(const char* name, cudaError_t failure = cudaErrorMemoryAllocation) {
@@ -45,6 +45,12 @@ int fake_calls(const char* name) {
     return g_calls[name];
 }
 int fake_null_launches() { return g_nullLaunches.exchange(0); }  // since the last call
+size_t fake_live_bytes() {  // of device memory
+    std::lock_guard<std::mutex> lock(g_mutex);
+    size_t sum = 0;
+    for (const auto& [p, n] : g_live) sum += n;
+    return sum;
+}
 // host memory that counts as page-locked
 void fake_page_locked(const void* p, size_t bytes) {
     std::lock_guard<std::mutex> lock(g_mutex);
@@ -59,10 +65,20 @@ const uint32_t gsr_logf_fixup_count = 0, gsr_logf_bucket_count = 1, gsr_logf_fix
 
 cudaError_t cudaMalloc(void** p, size_t n) {
     const cudaError_t e = called("cudaMalloc");
-    if (e == cudaSuccess) *p = std::aligned_alloc(256, (n + 255) / 256 * 256);
+    if (e != cudaSuccess) return e;
+    *p = std::aligned_alloc(256, (n + 255) / 256 * 256);
+    std::lock_guard<std::mutex> lock(g_mutex);
+    g_live[*p] = n;
     return e;
 }
-cudaError_t cudaFree(void* p) { std::free(p); return cudaSuccess; }
+cudaError_t cudaFree(void* p) {
+    {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        g_live.erase(p);
+    }
+    std::free(p);
+    return cudaSuccess;
+}
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
     const cudaError_t e = called("cudaHostAlloc");
     if (e == cudaSuccess) *p = std::malloc(n);

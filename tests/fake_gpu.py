@@ -30,6 +30,7 @@ def fake(fake_library, monkeypatch):
     lib = gsr_b200.load(build_if_missing=False)
     lib.fake_fail.argtypes = [C.c_char_p, C.c_int]
     lib.fake_page_locked.argtypes = [C.c_void_p, C.c_size_t]
+    lib.fake_live_bytes.restype = C.c_size_t
     yield lib
     for name in (b"cudaMalloc", b"cudaHostAlloc", b"cudaMemcpy", b"cudaMemcpyAsync", b"cudaStreamCreateWithFlags",
                  b"cudaEventCreateWithFlags"):

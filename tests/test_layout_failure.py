@@ -77,3 +77,28 @@ def test_the_old_layout_after_a_failure(fake):  # noqa: F811
         r.close()
     r.close()
     gs.close()
+
+
+@pytest.mark.parametrize("views", [1, 3])
+def test_a_sorted_layout_holds_no_row_wise_scratch(fake, views):  # noqa: F811
+    """Device memory of a sorted layout, against the global mode's: the depth sort's words and no more a
+    gaussian; after a row-wise layout in between the same again."""
+    count = 200_000
+    gs = gsr_b200.GpuScene(tile_raster_scene(count, seed=1))
+    start = fake.fake_live_bytes()
+    sorted_form, rows = _cams([(16, 4097)] * views), _cams([(640, 360)] * views)
+    held = {}
+    for mode in ("global", "binning"):
+        r = gsr_b200.Renderer(gs, gsr_b200.Settings(adaptive_list=False, list_mode=mode, budget_mb=8))
+        r.render_views(sorted_form)
+        held[mode] = fake.fake_live_bytes() - start
+        if mode == "binning":
+            r.render_views(rows)
+            assert fake.fake_live_bytes() - start > held[mode]
+            r.render_views(sorted_form)
+            assert fake.fake_live_bytes() - start == held[mode]
+        r.close()
+        assert fake.fake_live_bytes() == start
+    depth_sort = views * (count * 16 + 4 * -(-count // 4096) * 256 * 8 + 2 * 4 * 4 * 256)
+    assert held["binning"] - held["global"] < depth_sort + 64 * 1024
+    gs.close()
