@@ -18,7 +18,9 @@ the reference's real INRIA scenes are not available):
                    drawn from 0-3, 16 views at 3840x2160, learned colour with SH fallback
 
 `--config all` (the default) measures every workload; the line's headline `value` is the batched
-+ learned-colour form of learned_1080p (the metric's subject), `configs` holds each workload.
++ learned-colour form of learned_1080p (the metric's subject), `configs` holds each workload's rates.
+Everything else that was measured (pass times, parity, per-kernel rooflines, of every workload) goes to
+standard error as one JSON line before it.
 
 step         one pass over a workload's views: the 300-view orbit, the 64 batched views, the 16
              4K views. K steps are timed after W warm-up steps (at least until the adaptive
@@ -35,7 +37,8 @@ parity       per workload (the CPU leg, rank 0), one view (or one per resolution
              (keys, values, tile ranges) bit for bit against the oracle's construction, the
              float image's PSNR and the 8-bit image's PSNR and largest difference against the
              reference's own renderReference; forms that must equal another form say so.
-roofline     preprocess + sort (preprocess, depth sort, scan + emission, tile sort, ranges)
+roofline     preprocess + sort (preprocess, depth sort, scan + emission, tile sort, ranges; of a
+             list built by tile rows: the partition, then its tiles and ranges)
              against the measured HBM copy bandwidth: algorithmic bytes per frame over the
              summed CUDA-event pass times; each kernel's fraction in `kernels`. Measured on the
              headline's own frame (the batched form, its views per frame); `plain_view` holds
@@ -857,7 +860,7 @@ def view_checksums(r, frames: Frames, stream_obj) -> list[float]:
 
 
 def run_batched_64(G, args, dist, sampler, stream_obj):
-    """the 64 views one by one on the plain path (one renderer per resolution, so
+    """batched_64: the 64 views one by one on the plain path (one renderer per resolution, so
     no view changes a renderer's layout) against all of them in one frame."""
     scene, cams, fmt, layout, thr = workload("batched_64")
     mine = sharded(cams, dist)
@@ -931,7 +934,7 @@ def run_batched_64(G, args, dist, sampler, stream_obj):
 
 
 def run_scale_4k(G, args, dist, sampler, stream_obj, base_mem: int):
-    """16 4K views of 6M gaussians (fp16, per-gaussian degree), one by one and
+    """scale_4k: 16 4K views of 6M gaussians (fp16, per-gaussian degree), one by one and
     batched, plain SH and learned colour with SH fallback; peak device memory."""
     scene, cams, fmt, layout, thr = workload("scale_4k")
     mine = sharded(cams, dist)
@@ -1056,6 +1059,24 @@ def run_reference_arm(args):
 
 
 # ---- the B200 arm ---------------------------------------------------------------------------------
+def headline(line: dict) -> dict:
+    """What goes to standard output of everything measured: the line's own numbers, and of its nested
+    parts the few that say how the headline stands (a line of many kilobytes is cut by who reads it)."""
+    out = {k: v for k, v in line.items() if k not in ("config", "configs", "roofline", "render_issue", "issue", "render_flops",
+                                                      "parity")}
+    out["config"] = line["config"]
+    roof = line.get("roofline")
+    if roof:
+        out["roofline"] = {k: roof[k] for k in ("bound", "achieved", "peak", "unit", "frac", "peak_kind", "algorithmic_bytes",
+                                                "traffic") if k in roof}
+    parity = line.get("parity")
+    if parity:
+        out["parity"] = {k: parity[k] for k in ("list_bit_exact", "entries", "psnr_float_db", "psnr_8bit_db") if k in parity}
+    out["configs"] = {name: {form: r["views_per_s"] for form, r in forms.items() if isinstance(r, dict) and "views_per_s" in r}
+                      for name, forms in line["configs"].items()}
+    return out
+
+
 def run_b200(args, dist: Dist):
     import torch
 
@@ -1105,7 +1126,7 @@ def run_b200(args, dist: Dist):
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": head["ms_per_step"],
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": {"workload": workload_name, "gaussians": 1_240_000, "resolution": "1920x1080",
-                   "scene_format": "f32/soa", "bounds": "tight", "list": "adaptive, binning (depth sort + tile sort)",
+                   "scene_format": "f32/soa", "bounds": "tight", "list": "adaptive, binning (depth sort, then by tile rows)",
                    "form": form, "step": "one pass over the 300-view orbit (r=14, h=2)",
                    "l2": "inputs larger than L2 (scene 298 MB), no flush", "cuda_graph": True,
                    "parallelism": f"replicas x{dist.world} (orbit workloads); views split by pixel count "
@@ -1132,7 +1153,8 @@ def run_b200(args, dist: Dist):
                                             time_budget_s=30.0)
     line["wall_s"] = round(time.perf_counter() - t_start, 1)
     if dist.rank == 0:
-        print(json.dumps(line), flush=True)
+        print(json.dumps({"detail": line}), file=sys.stderr, flush=True)
+        print(json.dumps(headline(line)), flush=True)
 
 
 def main():
