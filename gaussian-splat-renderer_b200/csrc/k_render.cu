@@ -211,24 +211,6 @@ __device__ __forceinline__ float powerAt(const float4& u, const float4& w, float
     return fmaf(X, fmaf(u.x, X, fmaf(u.y, Y, u.w)), fmaf(Y, fmaf(u.z, Y, w.x), w.y));
 }
 
-// U entries of a hit list
-template <uint32_t U>
-__device__ __forceinline__ void loadHits(const uint32_t* hits, uint32_t (&q)[U]) {
-    if constexpr (U == 4) {
-        const uint4 v = *reinterpret_cast<const uint4*>(hits);
-        q[0] = v.x;
-        q[1] = v.y;
-        q[2] = v.z;
-        q[3] = v.w;
-    } else if constexpr (U == 2) {
-        const uint2 v = *reinterpret_cast<const uint2*>(hits);
-        q[0] = v.x;
-        q[1] = v.y;
-    } else {
-        q[0] = hits[0];
-    }
-}
-
 __device__ __forceinline__ uint32_t smemAddr(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
 // Four records (rows of the 2-D tensor map over the frame's record array: 12 fp32 columns, one
@@ -431,7 +413,7 @@ struct SlotWindow {
 // MODE: the record layout (kRenderSplatFull / P32 / P24), a compile-time parameter so that each
 // layout's kernel carries only its own gather and decode (a runtime switch measured 8 % slower).
 // CAP: 0, or the StopThePop window's register capacity; `ray` is then the shared area of the
-// gathered ray-depth parameters (3 x 16 B per entry, double-buffered).
+// gathered ray-depth parameters (RayArea: 36 bytes an entry, double-buffered).
 // TILE: the tile's code, 16 (INRIA's 16 x 16 tiles), 8 (8 x 8) or 32 (32 x 8); one or two pixels a
 // thread (pixelsPerThread), batches of one entry a thread, and each warp owns an 8 x 4 or 8 x 8 pixel
 // block of the tile (its strip: a squarer footprint meets fewer ellipses than a 16 x 2 row pair).
@@ -717,9 +699,10 @@ __device__ __forceinline__ void renderTile(const RenderArgs& a,
             if constexpr (CAP == 0 && !STATS) {
                 // PLAIN: every listed record's alpha is below the cap and its power never positive
                 auto walk = [&](auto plain) {
+                    static_assert(U == 2, "a group of hits is one 8-byte read");
                     for (uint32_t h = 0; h < listed; h += U) {
-                        uint32_t q[U];
-                        loadHits<U>(hits + h, q);
+                        const uint2 pair = *reinterpret_cast<const uint2*>(hits + h);
+                        const uint32_t q[U] = {pair.x, pair.y};
 #pragma unroll
                         for (uint32_t u = 0; u < U; ++u) {
                             const float4 pw0 = sm.power0[q[u]];

@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(kPartThreads, 4) rowPartitionKernel(const __gr
         const uint32_t view = t / perView, local = t - view * perView;
         const DevView vw = a.views[view];
         uint32_t listed = 0;
-        // the records' runs, four steps' loads in flight together
+        // the records' runs, the loads of kBatch steps in flight together
         auto forRuns = [&](auto fn) {
 #pragma unroll 1
             for (uint32_t s0 = 0; s0 < STEPS; s0 += kBatch) {

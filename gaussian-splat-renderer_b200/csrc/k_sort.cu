@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(kSortThreads, BITS == 9 ? 2 : 4) depthPassKern
 // a launch a pass and the look-backs, whose chain of latencies is what a sort this small spends its time
 // on (three passes over 10,000 words move 0.5 MB). Depth sort, one view, B200, us before / after: 1,000
 // records 29.0 / 14.7, 10,007 31.7 / 17.6, 30,000 32.4 / 24.1; the frames 78.2 / 65.4, 89.8 / 77.1,
-// 104.2 / 96.4. What bounds it now is the serial ranking of a warp's words and five block or cluster
+// 104.2 / 96.4. What bounds it now is the serial ranking of a warp's words and six block or cluster
 // barriers a pass.
 constexpr uint32_t kDepthClusterBlocks = 8;
 constexpr uint32_t kDepthClusterRecords = kDepthClusterBlocks * 4096;
