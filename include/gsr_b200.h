@@ -532,7 +532,10 @@ int gsr_read_image(GsrRenderer* r, float* rgba, uint8_t* rgb8);
 #define GSR_TILE_STAT_COUNT 8u
 int gsr_read_tile_stats(GsrRenderer* r, uint32_t* stats, uint32_t tiles, uint64_t* tested_pairs);
 /* Per-pass device time of the last frame in ms (GpuProfiler scopes), when timing is on: 5 passes
- * in global mode, 7 in binning mode (its front as preprocess, depth sort, scan + emission). */
+ * in global mode, 7 in binning mode (its front as preprocess, depth sort, scan + emission). The
+ * binning names are those of a sorted list; a list built by tile rows (GsrControl.ext_pad[0]) has
+ * its row plan and partition under "scan + duplicate (depth order)", its tiles and their ranges
+ * under "tile sort (total)", and about nothing under "tile ranges". */
 int gsr_renderer_set_timing(GsrRenderer* r, int enabled);
 int gsr_renderer_pass_times(GsrRenderer* r, float* ms, const char** names, uint32_t capacity, uint32_t* count);
 /* Capacity of the current list in entries, the budget's maximum, and list resizes so far. */
