@@ -853,6 +853,7 @@ __global__ void frameBeginKernel(DeviceControl* ctl, uint32_t count, uint32_t ca
         ctl->histDone[0] = 0;
         ctl->histDone[1] = 0;
         ctl->spillCursor = 0;
+        ctl->rowCutSlot = 0xFFFFFFFFu;
         ctl->rowTiles = 0;
         ctl->forceTimeout = forceTimeout;
     }

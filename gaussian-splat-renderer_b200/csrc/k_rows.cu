@@ -8,7 +8,8 @@
 //   rowPlan       one block: the rows' sizes, counted by the preprocess, into the places of their
 //                 buckets and of their tiles' part of the list. When the list overflows its capacity,
 //                 all blocks find the record it ends in (a scan of the counts in depth order) and
-//                 count the rows of the kept records instead.
+//                 count the rows of the kept records instead; they and the partition end at that record (four
+//                 720p views of 1.24 M, a capacity of 219,136: 286 -> 60 us; of 3.5 M: 333 -> 136)
 //   rowPartition  1,024 records a block in depth order: a row entry (x0, x1, gaussian) for every run
 //                 into its row's bucket, stable, with the onesweep sort's digit look-back (the digit is
 //                 the row)
@@ -293,7 +294,7 @@ __device__ void planRows(const FrontArgs& a, const unsigned long long* hist, uin
 
 __global__ void __launch_bounds__(kRowThreads) rowPlanKernel(const __grid_constant__ FrontArgs a) {
     __shared__ uint64_t sWarp[kRowWarps];
-    __shared__ uint32_t sTicket, sExclusive, sRows[kRowBins], sLast;
+    __shared__ uint32_t sTicket, sPast, sExclusive, sRows[kRowBins], sLast;
     __shared__ uint32_t sTerms[kRowWarps][kTermWords][32];
     gridWait();
     DeviceControl* ctl = a.ctl;
@@ -321,7 +322,6 @@ __global__ void __launch_bounds__(kRowThreads) rowPlanKernel(const __grid_consta
         c.sort_passes = a.totalTiles > 1 ? 1 : 0;  // (tile_max and key_bits: rowTiles)
         c.depth_low_bits = 0;
         c.sorted_buffer = 0;
-        if (!full) ctl->rowCutSlot = 0xFFFFFFFFu;
     }
     if (!full) {
         if (blockIdx.x == 0) planRows(a, a.rowHist, sWarp);
@@ -331,11 +331,19 @@ __global__ void __launch_bounds__(kRowThreads) rowPlanKernel(const __grid_consta
     const uint64_t* sorted = a.depthKeys[a.depthPlan->sortedBuffer & 1u];
     const uint32_t epoch = ctl->c.epoch, perView = (a.count + kRowTile - 1) / kRowTile;
     for (;;) {
-        if (tid == 0) sTicket = atomicAdd(&ctl->tickets[kRowCutTicket], 1u);
+        if (tid == 0) {
+            sTicket = atomicAdd(&ctl->tickets[kRowCutTicket], 1u);
+            sPast = __ldcg(&ctl->rowCutSlot) != 0xFFFFFFFFu;
+        }
         sRows[tid] = 0;
         __syncthreads();
         const uint32_t t = sTicket;
         if (t >= perView * a.viewCount) break;
+        if (sPast) {  // the cut lies before this tile (it is found after every tile up to it has published)
+            if (tid == 0) stRelaxed(&a.scanStatus[t], packStatus(epoch, kFlagInclusive, 0xFFFFFFFFu));
+            __syncthreads();
+            continue;
+        }
         const uint32_t view = t / perView, base = view * a.count + (t - view * perView) * kRowTile + tid * kRowSteps;
         const DevView vw = a.views[view];
         size_t rec[kRowSteps];
@@ -508,6 +516,7 @@ __global__ void __launch_bounds__(kPartThreads, 4) rowPartitionKernel(const __gr
         const uint32_t t = sTicket;
         if (t >= tiles) return;
         const uint32_t view = t / perView, local = t - view * perView;
+        if (view * a.count + local * kTile > cutSlot) return;  // past a full list's last record, as all tiles after it
         const DevView vw = a.views[view];
         uint32_t listed = 0;
         // the records' runs, the loads of kBatch steps in flight together
