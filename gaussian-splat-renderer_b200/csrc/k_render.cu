@@ -92,12 +92,16 @@ __host__ __device__ constexpr int tilePixels(int code) { return tileW(code) * ti
 // warps and strips. 1080p render pass 0.248 -> 0.196 ms, 24 uneven views 2.79 -> 1.87 ms, 4K 1.156
 // -> 0.873 ms. One pixel in 8 x 8 tiles (one warp a tile would have nothing to hide its latency),
 // with the window (its slots fill the registers) and in the stats build (its counts are a lane's).
+// One as well for the few tiles of a small image: they do not fill the chip, a tile's time is the
+// latency of its list's walk, and twice the warps hide it better. Render pass, two pixels / one (us):
+// 16 x 16 of 100,000 gaussians 3,078 / 1,596, 64 x 64 132 / 93, 256 x 256 (256 tiles) 56 / 44, 8192 x 16
+// (512) 2,494 / 1,227; two views of 256 x 256 of 1.24 M 107 / 92; medians over 2,000 to 1.24 M gaussians, near
+// and far: 256 tiles 0.85, 400 0.92, 512 0.94, 1,024 1.03, 1,900 1.10, 8,160 1.25 of two pixels.
+constexpr uint32_t kFewTiles = 512;
 __host__ __device__ constexpr int pixelsPerThread(int cap, int code, bool stats) {
     return cap == 0 && code != 8 && !stats ? 2 : 1;
 }
-__host__ __device__ constexpr int tileThreads(int cap, int code, bool stats) {
-    return tilePixels(code) / pixelsPerThread(cap, code, stats);
-}
+__host__ __device__ constexpr int tileThreads(int code, int px) { return tilePixels(code) / px; }
 
 // The warp strips (8 x 4 PX pixel blocks of a tile; bit w = warp w's) that a record's
 // cutoff ellipse q(d) = A dx^2 + 2B dx dy + C dy^2 <= t meets, computed once per record. At
@@ -425,15 +429,13 @@ struct SlotWindow {
 // blending and a record whose cutoff ellipse meets the pixel's warp strip).
 // GATHER: how the batch reaches shared memory (kGatherCpAsync or kGatherTma; TMA only with the
 // full records, no window and no statistics); map = the tensor map of the record array (TMA).
-template <int MODE, int CAP, int TILE, bool STATS, int GATHER>
-__device__ __forceinline__ void renderTile(const RenderArgs& a,
-                                           RenderShared<tileThreads(CAP, TILE, STATS), GATHER>& sm,
-                                           RayArea<tileThreads(CAP, TILE, STATS)>* ray, float4* slots,
+template <int MODE, int CAP, int TILE, bool STATS, int GATHER, int PX>
+__device__ __forceinline__ void renderTile(const RenderArgs& a, RenderShared<tileThreads(TILE, PX), GATHER>& sm,
+                                           RayArea<tileThreads(TILE, PX)>* ray, float4* slots,
                                            uint32_t tile, const CUtensorMap* map) {
     static_assert(GATHER == kGatherCpAsync || (MODE == kRenderSplatFull && CAP == 0 && !STATS), "the TMA gather");
     constexpr uint32_t kTW = tileW(TILE), kTH = tileH(TILE);
-    constexpr int PX = pixelsPerThread(CAP, TILE, STATS);
-    constexpr uint32_t kThreads = tileThreads(CAP, TILE, STATS), kStripW = 8, kRows = 4 * PX, kStripsX = kTW / kStripW;
+    constexpr uint32_t kThreads = tileThreads(TILE, PX), kStripW = 8, kRows = 4 * PX, kStripsX = kTW / kStripW;
     constexpr uint32_t U = CAP == 0 && !STATS ? kHitGroup : 1;  // hits of a warp whose alphas are computed together
     constexpr uint32_t kLanesX = kStripW / PX;  // lanes along a strip row, PX neighbouring pixels each
     static_assert(kThreads <= kRenderThreads && kThreads * PX == kTW * kTH && kTW % kStripW == 0 && kTH % kRows == 0,
@@ -901,26 +903,26 @@ __device__ __forceinline__ void initStage(RenderShared<N, GATHER>& sm) {
     }
 }
 
-template <int MODE, int CAP, int TILE, bool STATS, int GATHER>
-__global__ void __launch_bounds__(tileThreads(CAP, TILE, STATS), residentBlocks(CAP, tileThreads(CAP, TILE, STATS)))
+template <int MODE, int CAP, int TILE, bool STATS, int GATHER, int PX>
+__global__ void __launch_bounds__(tileThreads(TILE, PX), residentBlocks(CAP, tileThreads(TILE, PX)))
     renderKernel(const __grid_constant__ RenderArgs a, const __grid_constant__ CUtensorMap map) {
     extern __shared__ __align__(128) unsigned char smemRaw[];
-    constexpr int N = tileThreads(CAP, TILE, STATS);
+    constexpr int N = tileThreads(TILE, PX);
     RenderShared<N, GATHER>& sm = *reinterpret_cast<RenderShared<N, GATHER>*>(smemRaw);
     initStage(sm);
     gridWait();
-    renderTile<MODE, CAP, TILE, STATS, GATHER>(a, sm, CAP > 0 ? rayArea<N, GATHER>(smemRaw) : nullptr,
-                                               CAP > 0 ? slotArea<N, GATHER>(smemRaw) : nullptr,
-                                               blockIdx.x + a.tileOffset, &map);
+    renderTile<MODE, CAP, TILE, STATS, GATHER, PX>(a, sm, CAP > 0 ? rayArea<N, GATHER>(smemRaw) : nullptr,
+                                                   CAP > 0 ? slotArea<N, GATHER>(smemRaw) : nullptr,
+                                                   blockIdx.x + a.tileOffset, &map);
 }
 
 // Persistent schedule: each block takes tiles from the frame's queue counter (reset by frame
 // begin) until the counter passes the last tile.
-template <int MODE, int CAP, int TILE, bool STATS, int GATHER>
-__global__ void __launch_bounds__(tileThreads(CAP, TILE, STATS), residentBlocks(CAP, tileThreads(CAP, TILE, STATS)))
+template <int MODE, int CAP, int TILE, bool STATS, int GATHER, int PX>
+__global__ void __launch_bounds__(tileThreads(TILE, PX), residentBlocks(CAP, tileThreads(TILE, PX)))
     renderPersistentKernel(const __grid_constant__ RenderArgs a, const __grid_constant__ CUtensorMap map) {
     extern __shared__ __align__(128) unsigned char smemRaw[];
-    constexpr int N = tileThreads(CAP, TILE, STATS);
+    constexpr int N = tileThreads(TILE, PX);
     RenderShared<N, GATHER>& sm = *reinterpret_cast<RenderShared<N, GATHER>*>(smemRaw);
     initStage(sm);
     gridWait();
@@ -929,24 +931,24 @@ __global__ void __launch_bounds__(tileThreads(CAP, TILE, STATS), residentBlocks(
         __syncthreads();
         const uint32_t tile = sm.tile;
         if (tile >= a.totalTiles) break;
-        renderTile<MODE, CAP, TILE, STATS, GATHER>(a, sm, CAP > 0 ? rayArea<N, GATHER>(smemRaw) : nullptr,
-                                               CAP > 0 ? slotArea<N, GATHER>(smemRaw) : nullptr,
-                                                   tile, &map);
+        renderTile<MODE, CAP, TILE, STATS, GATHER, PX>(a, sm, CAP > 0 ? rayArea<N, GATHER>(smemRaw) : nullptr,
+                                                       CAP > 0 ? slotArea<N, GATHER>(smemRaw) : nullptr,
+                                                       tile, &map);
         __syncthreads();  // every thread has read sm.tile and left the tile's shared buffers
     }
 }
 
-template <int MODE, int CAP, int TILE, bool STATS = false, int GATHER = kGatherCpAsync>
+template <int MODE, int CAP, int TILE, bool STATS = false, int GATHER = kGatherCpAsync, int PX = pixelsPerThread(CAP, TILE, STATS)>
 cudaError_t launchRenderMode(const RenderArgs& a, cudaStream_t s) {
-    constexpr uint32_t threads = tileThreads(CAP, TILE, STATS);
-    constexpr size_t smem = renderSmemBytes<CAP, tileThreads(CAP, TILE, STATS), GATHER>();
+    constexpr uint32_t threads = tileThreads(TILE, PX);
+    constexpr size_t smem = renderSmemBytes<CAP, int(threads), GATHER>();
     static std::atomic<bool> configuredOn[64] = {};
     std::atomic<bool>& configured = perDevice(configuredOn);
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(renderKernel<MODE, CAP, TILE, STATS, GATHER>,
+        cudaError_t e = cudaFuncSetAttribute(renderKernel<MODE, CAP, TILE, STATS, GATHER, PX>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(renderPersistentKernel<MODE, CAP, TILE, STATS, GATHER>,
+        e = cudaFuncSetAttribute(renderPersistentKernel<MODE, CAP, TILE, STATS, GATHER, PX>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;
         configured = true;
@@ -958,10 +960,10 @@ cudaError_t launchRenderMode(const RenderArgs& a, cudaStream_t s) {
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         // as many resident threads per SM for either tile size
         const uint32_t grid = uint32_t(sms) * kPersistentBlocksPerSm * (kRenderThreads / threads);
-        return launchDependent(renderPersistentKernel<MODE, CAP, TILE, STATS, GATHER>,
+        return launchDependent(renderPersistentKernel<MODE, CAP, TILE, STATS, GATHER, PX>,
                                dim3(grid < a.totalTiles ? grid : a.totalTiles), threads, smem, s, a, map);
     }
-    return launchDependent(renderKernel<MODE, CAP, TILE, STATS, GATHER>, dim3(a.tileLaunch ? a.tileLaunch : a.totalTiles),
+    return launchDependent(renderKernel<MODE, CAP, TILE, STATS, GATHER, PX>, dim3(a.tileLaunch ? a.tileLaunch : a.totalTiles),
                            threads, smem, s, a, map);
 }
 
@@ -970,10 +972,14 @@ cudaError_t launchRenderMode(const RenderArgs& a, cudaStream_t s) {
 template <int MODE, int TILE>
 cudaError_t launchRenderWindow(const RenderArgs& a, cudaStream_t s) {
     if (a.tileStats) return launchRenderMode<MODE, 0, TILE, true>(a, s);  // the stats build has no window
+    const bool few = (a.tileLaunch ? a.tileLaunch : a.totalTiles) <= kFewTiles;
     if constexpr (MODE == kRenderSplatFull) {
-        if (a.sortWindow == 0 && a.splatMap) return launchRenderMode<MODE, 0, TILE, false, kGatherTma>(a, s);
+        if (a.sortWindow == 0 && a.splatMap)
+            return few ? launchRenderMode<MODE, 0, TILE, false, kGatherTma, 1>(a, s)
+                       : launchRenderMode<MODE, 0, TILE, false, kGatherTma>(a, s);
     }
-    if (a.sortWindow == 0) return launchRenderMode<MODE, 0, TILE>(a, s);
+    if (a.sortWindow == 0)
+        return few ? launchRenderMode<MODE, 0, TILE, false, kGatherCpAsync, 1>(a, s) : launchRenderMode<MODE, 0, TILE>(a, s);
     if (a.sortWindow <= 4) return launchRenderMode<MODE, 4, TILE>(a, s);
     if (a.sortWindow <= 8) return launchRenderMode<MODE, 8, TILE>(a, s);
     if (a.sortWindow <= 16) return launchRenderMode<MODE, 16, TILE>(a, s);
