@@ -96,8 +96,10 @@ __host__ __device__ constexpr int tilePixels(int code) { return tileW(code) * ti
 // latency of its list's walk, and twice the warps hide it better. Render pass, two pixels / one (us):
 // 16 x 16 of 100,000 gaussians 3,078 / 1,596, 64 x 64 132 / 93, 256 x 256 (256 tiles) 56 / 44, 8192 x 16
 // (512) 2,494 / 1,227; two views of 256 x 256 of 1.24 M 107 / 92; medians over 2,000 to 1.24 M gaussians, near
-// and far: 256 tiles 0.85, 400 0.92, 512 0.94, 1,024 1.03, 1,900 1.10, 8,160 1.25 of two pixels.
-constexpr uint32_t kFewTiles = 512;
+// and far: 256 tiles 0.85, 400 0.92, 512 0.94, 1,024 1.03, 1,900 1.10, 8,160 1.25 of two pixels. From 65,536
+// gaussians on, whose lists are longer, up to 1,024 tiles: 640 x 360 (920) of 300,000 gaussians 0.72 far, 0.91
+// from 1.75 radii, 1.04 near; of 1.24 M 0.67, 0.77, 1.11; at 1,200 tiles 0.89, 0.95, 1.08 and 0.68, 0.87, 1.14.
+constexpr uint32_t kFewTiles = 512, kFewTilesLong = 1024, kLongCount = 65536;
 __host__ __device__ constexpr int pixelsPerThread(int cap, int code, bool stats) {
     return cap == 0 && code != 8 && !stats ? 2 : 1;
 }
@@ -972,7 +974,7 @@ cudaError_t launchRenderMode(const RenderArgs& a, cudaStream_t s) {
 template <int MODE, int TILE>
 cudaError_t launchRenderWindow(const RenderArgs& a, cudaStream_t s) {
     if (a.tileStats) return launchRenderMode<MODE, 0, TILE, true>(a, s);  // the stats build has no window
-    const bool few = (a.tileLaunch ? a.tileLaunch : a.totalTiles) <= kFewTiles;
+    const bool few = (a.tileLaunch ? a.tileLaunch : a.totalTiles) <= (a.count < kLongCount ? kFewTiles : kFewTilesLong);
     if constexpr (MODE == kRenderSplatFull) {
         if (a.sortWindow == 0 && a.splatMap)
             return few ? launchRenderMode<MODE, 0, TILE, false, kGatherTma, 1>(a, s)

@@ -57,3 +57,15 @@ def test_forms(gpu, kw, tile):
     gs = gpu.GpuScene(_scene(3000, False))
     assert _images(gpu, gs, [cam], 1, tile_size=tile, **kw)[0] == _images(gpu, gs, [cam] * 20, 20, tile_size=tile, **kw)[1]
     gs.close()
+
+
+def test_the_line_of_many_gaussians(gpu):
+    """1,024 and 1,025 tiles of 65,536 gaussians."""
+    from gsr_b200 import scenes
+
+    gs = gpu.GpuScene(_scene(65_536, False))
+    cams = [scenes.viewer_camera((0.3, 0.5, 6.0), (0.0, 0.0, 0.0), 512, 512, 30.0),
+            scenes.viewer_camera((0.3, 0.5, 6.0), (0.0, 0.0, 0.0), 9, 16, 30.0)]
+    for views in (1, 2):
+        assert _images(gpu, gs, cams, views) == _images(gpu, gs, cams, views, tile_stats=True)
+    gs.close()
