@@ -603,13 +603,18 @@ struct GsrRenderer {
     // 2,370 against 2,381; up to 384 rows 0.76 to 1.14 of the sorted list. The line lies lower with
     // small tiles, of which a splat has more to sort (30,000 in 8 views of 1280 x 720, 8-px tiles: 491
     // against 513), and higher with 32 x 8 ones (60,000: 625 against 606).
+    // Nor, for many records, views much higher than wide, whose rows' runs are hardly fewer than their tiles
+    // (1.24 M at 16 x 4096, near: 620 against 320; at 128 x 4096 673 against 450; at 1080 x 1920 as fast as at
+    // 1920 x 1080), or a single tile, which eight blocks fill (100,000: 98 against 75).
     bool rowWiseFits(uint32_t v) const {
         const uint32_t few = settings.tile_size == 8 ? 20000u : settings.tile_size == 16 ? 40000u : 65000u;
-        return binning() && maxTilesY <= kRowBins && maxTilesX <= kRowMaxTilesX &&
-               uint64_t(scene.count) * v <= kRowMaxRecords * totalRows && (totalRows <= kRowFewRows || scene.count > few);
+        const uint64_t records = uint64_t(scene.count) * v;
+        return binning() && maxTilesY <= kRowBins && maxTilesX <= kRowMaxTilesX && records <= kRowMaxRecords * totalRows &&
+               (totalRows <= kRowFewRows || scene.count > few) && records <= kRowMany * totalTiles &&
+               (maxTilesY <= 8 * maxTilesX || scene.count <= kRowMany);
     }
     uint64_t totalRows = 0;
-    static constexpr uint64_t kRowMaxRecords = 196608, kRowFewRows = 384;
+    static constexpr uint64_t kRowMaxRecords = 196608, kRowFewRows = 384, kRowMany = 65536;
     uint32_t rowHistWords() const { return allocViews * kRowBins * 2 * 2; }
     uint32_t rowStatusVec4s(uint32_t v) const {
         const uint64_t tile = rowPartitionTile(uint64_t(scene.count) * v);

@@ -58,15 +58,15 @@ def test_a_row_past_32_bits(gpu):
 
 def test_more_spilled_runs_than_32_bits_count(gpu):
     """17.2 M needles over all 256 tile rows ask for 4.4 G spilled runs; the near half, of which the list's
-    records are, is in the image's second tile column, the far half in its third."""
+    records are, is in the image's 16th tile column, the far half in its 17th."""
     count = 17_200_000
     x = np.where(np.arange(count) < count // 2, -0.009, 0.0135)
     scene = _scene(count, x, (0.001, 20.0, 0.001), 0.5)
-    hi, val, ranges, cap = _frame(gpu, scene, 64, 4096, "tight")
+    hi, val, ranges, cap = _frame(gpu, scene, 512, 4096, "tight")
     of_row = cap // 256 + (np.arange(256) < cap % 256)
     end = np.cumsum(of_row)
-    want = np.zeros((256, 4, 2), np.uint32)
-    want[:, 1] = np.stack([end - of_row, end], 1)
+    want = np.zeros((256, 32, 2), np.uint32)
+    want[:, 15] = np.stack([end - of_row, end], 1)
     np.testing.assert_array_equal(ranges, want.reshape(-1, 2))
-    np.testing.assert_array_equal(hi, np.repeat(np.arange(256) * 4 + 1, of_row))
+    np.testing.assert_array_equal(hi, np.repeat(np.arange(256) * 32 + 15, of_row))
     np.testing.assert_array_equal(val, np.arange(cap) - np.repeat(end - of_row, of_row))

@@ -9,10 +9,10 @@ from helpers import tile_raster_scene
 pytestmark = pytest.mark.gpu
 
 
-def _cams(views):
+def _cams(views, size=(256, 128)):
     from gsr_b200 import scenes
 
-    return [scenes.viewer_camera((7.0 * np.sin(k), 0.5, 7.0 * np.cos(k)), (0.0, 0.0, 0.0), 256, 128, 60.0)
+    return [scenes.viewer_camera((7.0 * np.sin(k), 0.5, 7.0 * np.cos(k)), (0.0, 0.0, 0.0), *size, 60.0)
             for k in range(views)]
 
 
@@ -40,6 +40,23 @@ def test_the_line(gpu, count, views, tile, row_wise):
                 frame, rows = _frame(r, cams[:views_now])
                 assert rows == (row_wise if views_now == views else True)
             frames.append(frame)
+        r.close()
+    for a, b in zip(*frames):
+        np.testing.assert_array_equal(a, b)
+    gs.close()
+
+
+@pytest.mark.parametrize("count,size,views,row_wise", [
+    (65_536, (16, 16), 1, True), (65_537, (16, 16), 1, False), (65_537, (17, 16), 1, True),
+    (65_536, (32, 300), 1, True), (65_537, (32, 256), 1, True), (65_537, (32, 257), 2, False), (65_537, (33, 257), 1, True)])
+def test_single_tiles_and_high_views(gpu, count, size, views, row_wise):
+    gs = gpu.GpuScene(tile_raster_scene(count, seed=6))
+    frames = []
+    for mode in ("binning", "global"):
+        r = gpu.Renderer(gs, gpu.Settings(adaptive_list=False, list_mode=mode, budget_mb=1024))
+        frame, rows = _frame(r, _cams(views, size))
+        assert rows == (row_wise and mode == "binning")
+        frames.append(frame)
         r.close()
     for a, b in zip(*frames):
         np.testing.assert_array_equal(a, b)
