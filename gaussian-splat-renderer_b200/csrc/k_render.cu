@@ -2,8 +2,8 @@
 // the CPU reference's per-pixel loop, src/splat/reference_renderer.cpp:120-222).
 //
 // One 128-thread block per 16x16 tile, two neighbouring pixels a thread; warp w owns an 8 x 8 pixel
-// block. (The window, the stats build and 8 x 8 tiles: one pixel a thread, 8 x 4 blocks.) The tile's
-// entries [ranges[tile].x, ranges[tile].y) are walked front to back in batches of one record a
+// block. (The window, the stats build, 8 x 8 tiles and launches of few tiles: one pixel a thread, 8 x 4
+// blocks.) The tile's entries [ranges[tile].x, ranges[tile].y) are walked front to back in batches of one record a
 // thread: while batch b is blended, the records of batch b+1 are gathered into shared memory with
 // cp.async (16-byte LDGSTS, the record of gaussian values[j], each thread its own). Each
 // entry is then prepared once per block: its power, in base 2 and with log2(opacity) added,
