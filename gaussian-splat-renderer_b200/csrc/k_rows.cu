@@ -9,7 +9,7 @@
 //                 buckets and of their tiles' part of the list. When the list overflows its capacity,
 //                 all blocks find the record it ends in (a scan of the counts in depth order) and
 //                 count the rows of the kept records instead; they and the partition end at that record (four
-//                 720p views of 1.24 M, a capacity of 219,136: 286 -> 60 us; of 3.5 M: 333 -> 136)
+//                 720p views of 1.24 M, a capacity of 219,136: 286 -> 79 us; of 3.5 M: 333 -> 153)
 //   rowPartition  1,024 records a block in depth order: a row entry (x0, x1, gaussian) for every run
 //                 into its row's bucket, stable, with the onesweep sort's digit look-back (the digit is
 //                 the row)
@@ -292,6 +292,40 @@ __device__ void planRows(const FrontArgs& a, const unsigned long long* hist, uin
     if (threadIdx.x == 0) a.ctl->c.ext_pad[0] = uint32_t(total >> 32);  // the row entries
 }
 
+// A full list's largest tile id is that of all records, kept or not: the end of the longest run in the last
+// row with tiles, found by all blocks together from the view's hints as they lie (16 bytes a record; 1.24 M: 17
+// us).
+__device__ void reportLastTile(const FrontArgs& a, uint32_t view, uint32_t row) {
+    const DevView vw = a.views[view];
+    uint32_t end = 0;
+    for (uint32_t i0 = blockIdx.x * kRowTile + threadIdx.x; i0 < a.count; i0 += gridDim.x * kRowTile) {
+        size_t rec[kRowSteps];
+        uint32_t kept[kRowSteps];
+        RecordRows R[kRowSteps];
+#pragma unroll
+        for (uint32_t j = 0; j < kRowSteps; ++j) {
+            const uint32_t i = i0 + j * kRowThreads;
+            rec[j] = size_t(view) * a.count + (i < a.count ? i : 0u);
+            kept[j] = i < a.count ? a.tileCounts[rec[j]] : 0u;
+        }
+        recordRows(a, vw, rec, kept, R);
+#pragma unroll
+        for (uint32_t j = 0; j < kRowSteps; ++j) {
+            const uint32_t r = row - R[j].r0;
+            if (kept[j] && r < R[j].rows) {
+                const uint32_t run = runOf(a, vw, rec[j], R[j].r0, r, R[j].at, R[j].run[0]);
+                if ((run >> 16) > (run & 0xFFFFu) && (run >> 16) <= vw.tilesX) end = end > (run >> 16) ? end : run >> 16;
+            }
+        }
+    }
+    end = __reduce_max_sync(0xFFFFFFFFu, end);
+    if ((threadIdx.x & 31) == 0 && end && row < vw.tilesY) {
+        const uint32_t tile = vw.tileBase + row * vw.tilesX + end - 1;
+        atomicMax(&a.ctl->c.tile_max, tile);
+        atomicMax(&a.ctl->c.key_bits, bitWidth32(tile));
+    }
+}
+
 __global__ void __launch_bounds__(kRowThreads) rowPlanKernel(const __grid_constant__ FrontArgs a) {
     __shared__ uint64_t sWarp[kRowWarps];
     __shared__ uint32_t sTicket, sPast, sExclusive, sRows[kRowBins], sLast;
@@ -301,12 +335,16 @@ __global__ void __launch_bounds__(kRowThreads) rowPlanKernel(const __grid_consta
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // every block adds up the frame's tiles from the rows' low words, unless one of them may have gone past
     // 2^32 and carried into its entries (which are not read then: a full list is planned from its kept records)
-    uint64_t sum = 0, all = ctl->rowTiles;
-    if (!a.rowTilesWide) {
+    uint64_t sum = 0, all;
+    uint32_t lastRow = 0;  // the last bucket with tiles
 #pragma unroll 8
-        for (uint32_t j = tid; j < a.viewCount * kRowBins; j += kRowThreads) sum += __ldcg(&a.rowHist[j]) & 0xFFFFFFFFull;
-        blockScan64(sum, sWarp, &all);
+    for (uint32_t j = tid; j < a.viewCount * kRowBins; j += kRowThreads) {
+        const uint64_t h = __ldcg(&a.rowHist[j]);
+        sum += h & 0xFFFFFFFFull;
+        if (h) lastRow = j;
     }
+    blockScan64(sum, sWarp, &all);
+    if (a.rowTilesWide) all = ctl->rowTiles;
     const uint32_t tiles = uint32_t(all < 0xFFFFFFFFull ? all : 0xFFFFFFFFull);
     const bool full = tiles > a.capacity;
     if (blockIdx.x == 0 && tid == 0) {
@@ -327,6 +365,11 @@ __global__ void __launch_bounds__(kRowThreads) rowPlanKernel(const __grid_consta
         if (blockIdx.x == 0) planRows(a, a.rowHist, sWarp);
         return;
     }
+    if (tid == 0) sLast = 0;
+    __syncthreads();
+    atomicMax(&sLast, lastRow);
+    __syncthreads();
+    reportLastTile(a, sLast / kRowBins, sLast % kRowBins);
     // the list ends inside the record at which the counts' prefix in depth order reaches the capacity
     const uint64_t* sorted = a.depthKeys[a.depthPlan->sortedBuffer & 1u];
     const uint32_t epoch = ctl->c.epoch, perView = (a.count + kRowTile - 1) / kRowTile;
