@@ -18,7 +18,7 @@ def fake_library(tmp_path_factory):
     csrc = REPO / "gaussian-splat-renderer_b200" / "csrc"
     subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-pthread", f"-I{REPO / 'include'}", f"-I{csrc}",
                     f"-I{CUDA / 'include'}", "-o", out, csrc / "renderer.cpp", csrc / "color_checkpoint.cpp",
-                    REPO / "tests" / "fake_gpu.cpp", "-Wl,-z,defs"], check=True)
+                    REPO / "tests" / "fake_gpu.cpp", "-Wl,-z,defs,-Bsymbolic"], check=True)
     return out
 
 
