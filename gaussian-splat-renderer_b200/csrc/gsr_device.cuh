@@ -54,6 +54,11 @@ __device__ __forceinline__ bool statusReady(uint64_t s, uint32_t epoch) {
 }
 __device__ __forceinline__ uint64_t statusFlag(uint64_t s) { return (s >> 32) & 3u; }
 
+static_assert(alignof(DeviceControl) == 4 && offsetof(DeviceControl, rowTiles) % 8 == 0, "the block's two words of tiles");
+__device__ __forceinline__ unsigned long long* rowTilesOf(DeviceControl* ctl) {  // (the block is at an allocation's start)
+    return reinterpret_cast<unsigned long long*>(ctl->rowTiles);
+}
+
 __device__ __forceinline__ void reportTimeout(DeviceControl* ctl, uint32_t where) {
     atomicOr(&ctl->c.status, uint32_t(GSR_CONTROL_TIMEOUT));
     atomicExch(&ctl->c.timeout_where, where);

@@ -614,7 +614,7 @@ __global__ void __launch_bounds__(kFrontThreads, 4) preprocessKernel(const __gri
     if (a.rowRecords && sRows[tid])
         atomicAdd(&a.rowHist[size_t(view) * kRowBins + tid],
                   (static_cast<unsigned long long>(sRows[tid] >> 20) << 32) | (sRows[tid] & 0xFFFFFu));
-    if (a.rowTilesWide && tid == 0 && sTiles) atomicAdd(&a.ctl->rowTiles, static_cast<unsigned long long>(sTiles));
+    if (a.rowTilesWide && tid == 0 && sTiles) atomicAdd(rowTilesOf(a.ctl), static_cast<unsigned long long>(sTiles));
     if (tid < kCullReasonCount && sCull[tid]) atomicAdd(&a.ctl->c.cull_counts[tid], sCull[tid]);
     if (tid == 0 && sDepthMin <= sDepthMax) {
         atomicMin(&a.ctl->c.depth_min_bits, sDepthMin);
@@ -854,7 +854,7 @@ __global__ void frameBeginKernel(DeviceControl* ctl, uint32_t count, uint32_t ca
         ctl->histDone[1] = 0;
         ctl->spillCursor = 0;
         ctl->rowCutSlot = 0xFFFFFFFFu;
-        ctl->rowTiles = 0;
+        ctl->rowTiles[0] = ctl->rowTiles[1] = 0;
         ctl->forceTimeout = forceTimeout;
     }
 }

@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(kRowThreads) rowPlanKernel(const __grid_consta
         if (h) lastRow = j;
     }
     blockScan64(sum, sWarp, &all);
-    if (a.rowTilesWide) all = ctl->rowTiles;
+    if (a.rowTilesWide) all = *rowTilesOf(ctl);
     const uint32_t tiles = uint32_t(all < 0xFFFFFFFFull ? all : 0xFFFFFFFFull);
     const bool full = tiles > a.capacity;
     if (blockIdx.x == 0 && tid == 0) {
